@@ -240,7 +240,15 @@ static const int2* kp_tiles(lapw1gpu_kpoint* k, const std::string& key, int* cou
     cudaGetLastError();
     return nullptr;
   }
-  if (cudaMemcpy(d, t.data(), sizeof(int2) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+  // The list must be on the device before any stream's kernel reads it: a
+  // plain cudaMemcpy of up to 64 KB from pageable memory returns while its
+  // copy is still queued on the legacy stream, which the context's
+  // non-blocking streams do not wait for.  The last chain's stream is idle
+  // in all but four-chain batches, so waiting for it waits for the copy.
+  cudaStream_t cs = k->ctx->side[L1G_MAX_SETS - 1];
+  if (cudaMemcpyAsync(d, t.data(), sizeof(int2) * t.size(), cudaMemcpyHostToDevice, cs) != cudaSuccess ||
+      cudaStreamSynchronize(cs) != cudaSuccess) {
+    cudaGetLastError();
     cudaFree(d);
     return nullptr;
   }
