@@ -22,11 +22,24 @@
 // gathered from the Theta/WARP table and HS is written as k_spherical does.
 //
 // Warp roles: warps 0..4 EG-1 epilogue (warp w reads TMEM lanes 32 (w%4)..
-// and the I group w/4 of 4 I), warp 4 EG lane 0 issues the MMAs, warp
-// 4 EG + 1 lane 0 the TMA loads (a full ring ahead of the MMAs, whatever
-// they wait on).  Every
+// and the I group w/4 of 4 I), warp 4 EG issues the MMAs, warp 4 EG + 1 lane 0
+// the TMA loads (a full ring ahead of the MMAs, whatever they wait on).  Every
 // mbarrier wait is bounded; a timeout sets a status bit and ends the CTA's
 // work cleanly (copies drained, MMAs complete, TMEM freed).
+//
+// What bounds it (clock sums of the roles, 5 slices): at 100 atoms (13 K steps
+// per l) the tensor core, about 60% of the kernel, and the operand feed that
+// it waits for the rest of the time; at 40 atoms (5 K steps) MMAs, feed and
+// epilogue about equally.  Issued by one lane in a branch of its own, an MMA
+// took 110 clocks of that lane against 77 on the tensor core, and the scales
+// of the epilogue (Legendre weight, exponents) 580 clocks per pair and l
+// behind the TMEM loads; with the issue from a converged warp, the scales
+// formed before the wait for the accumulator, explicit polynomials and the
+// tile's rows in shared memory, 40 atoms (N = 4937) went from 1.69 to 1.37 ms
+// and 100 atoms (N = 12677) from 22.0 to 19.4 ms (38.0 to 33.1 Mclk; the power
+// cap then lowers the clock).  A tile of two 12-I halves that share each A
+// block (36% less feed, 8 pairs per epilogue thread by a register split) took
+// the same time and was not kept, nor did row pitches of 64 or 128 bytes help.
 #pragma once
 
 namespace sphtc {
@@ -34,12 +47,15 @@ namespace sphtc {
 using split::desc_kblock;
 using split::digit7;
 using split::digit_scale;
+using split::elect_one;
 using split::i2d_exact;
 using split::idesc_i8;
 using split::mbar_expect_tx;
 using split::mbar_init;
 using split::mbar_try_wait;
 using split::mbar_wait;
+using split::mma_commit;
+using split::mma_i8;
 using split::smem_u32;
 using split::tc_fence_after;
 using split::tc_fence_before;
@@ -66,13 +82,16 @@ struct Cfg {
   static constexpr int KSTEPS = KB / 32;  // 32-byte MMA K steps per stage
   static constexpr int A_BYTES = S * 128 * KB;
   static constexpr int B_BYTES = S * N * KB;
-  static constexpr int STAGE = A_BYTES + B_BYTES;
-  // per-tile exponent tables: eA - 12 per (l, J) and eB per (l, I, S|H), int16
+  // per-tile tables: exponents eA - 12 per (l, J) and eB per (l, I, S|H) as
+  // int16, and the rows of the tile's I (unit vector, length, KZZ)
   static constexpr int SCALE_BYTES = (SPH_LMAX * 128 + SPH_LMAX * 2 * IT) * 2;
-  static constexpr int STAGES_FIT = (227 * 1024 - SCALE_BYTES - 1024) / STAGE;
+  static constexpr int ROW_BYTES = IT * 48;
+  static constexpr int ROOM = 227 * 1024 - SCALE_BYTES - ROW_BYTES - 1024;
+  static constexpr int STAGE = A_BYTES + B_BYTES;
+  static constexpr int STAGES_FIT = ROOM / STAGE;
   static constexpr int STAGES = STAGES_FIT > 8 ? 8 : STAGES_FIT;
   static_assert(STAGES >= 2, "the ring needs two stages");
-  static constexpr int SMEM = STAGES * STAGE + SCALE_BYTES + 1024;
+  static constexpr int SMEM = STAGES * STAGE + SCALE_BYTES + ROW_BYTES + 1024;
   static constexpr int THREADS = EPI + 64;  // + the MMA warp and the TMA warp
 };
 
@@ -182,9 +201,84 @@ __global__ void __launch_bounds__(256, 2) k_sph_slice(DevProb P, const SphCoef* 
 // 2^e as a double from its exponent bits: exact for -1022 <= e <= 1023,
 // 0 below that range and infinity above it (no branch)
 __device__ __forceinline__ double pow2i(int e) {
-  const double v = __longlong_as_double((long long)(min(max(e, -1023), 1024) + 1023) << 52);
-  return e < -1022 ? 0.0 : v;
+  return __hiloint2double((min(max(e, -1023), 1024) + 1023) << 20, 0);  // biased exponent 0: the double 0
 }
+
+// Coefficients of (2l+1) P_l(x) by descending power: x^(l odd) times a
+// polynomial of degree l/2 in x^2, P_l = 2^-l sum_k (-1)^k C(l,k) C(2l-2k,l) x^(l-2k)
+struct LegCoef {
+  double c[SPH_LMAX][(SPH_LMAX + 1) / 2];
+};
+__host__ __device__ constexpr LegCoef leg_make() {
+  LegCoef t{};
+  for (int l = 0; l < SPH_LMAX; l++)
+    for (int k = 0; k <= l / 2; k++) {
+      double v = 1.0;
+      for (int i = 1; i <= k; i++) v = v * (l - k + i) / i;      // C(l,k)
+      double w = 1.0;
+      for (int i = 1; i <= l; i++) w = w * (l - 2 * k + i) / i;  // C(2l-2k,l)
+      double q = (k & 1) ? -v * w : v * w;
+      for (int i = 0; i < l; i++) q *= 0.5;
+      t.c[l][k] = q * (2 * l + 1);
+    }
+  return t;
+}
+template <int l, int N>
+__device__ __forceinline__ void leg_poly(const double (&x)[N], double (&w)[N]) {
+  constexpr LegCoef K = leg_make();
+#pragma unroll
+  for (int u = 0; u < N; u++) {
+    const double t = x[u] * x[u];
+    double p = K.c[l][0];
+#pragma unroll
+    for (int k = 1; k <= l / 2; k++) p = fma(p, t, K.c[l][k]);
+    w[u] = (l & 1) ? p * x[u] : p;
+  }
+}
+// w = (2l+1) P_l(x) of N pairs from the explicit polynomials: independent
+// chains with the coefficients as constant operands, and no values of the
+// orders below l to keep.  Rounding: at most eps sum |c_k|, 1e-12 at l = 12
+// near |x| = 1 and below 2e-13 up to l = 10, under the slice products' error
+// at 5 slices (2e-10).  line: bits of the pairs along one line, which take
+// x P_(l-1) at every order (hamilt.F:250-281), so x^l.
+template <int N>
+__device__ __forceinline__ void leg_weights(int l, const double (&x)[N], unsigned line, double (&w)[N]) {
+  switch (l) {
+    case 0: leg_poly<0>(x, w); break;
+    case 1: leg_poly<1>(x, w); break;
+    case 2: leg_poly<2>(x, w); break;
+    case 3: leg_poly<3>(x, w); break;
+    case 4: leg_poly<4>(x, w); break;
+    case 5: leg_poly<5>(x, w); break;
+    case 6: leg_poly<6>(x, w); break;
+    case 7: leg_poly<7>(x, w); break;
+    case 8: leg_poly<8>(x, w); break;
+    case 9: leg_poly<9>(x, w); break;
+    case 10: leg_poly<10>(x, w); break;
+    case 11: leg_poly<11>(x, w); break;
+    default: leg_poly<12>(x, w); break;
+  }
+  static_assert(SPH_LMAX == 13, "one case per order");
+  if (line) {
+#pragma unroll
+    for (int u = 0; u < N; u++)
+      if ((line >> u) & 1) {
+        double p = (double)(2 * l + 1);
+        for (int k = 0; k < l; k++) p *= x[u];
+        w[u] = p;
+      }
+  }
+}
+// (l-1)/l of the Legendre recursion
+struct LegRatio {
+  double c[SPH_LMAX];
+};
+constexpr LegRatio leg_ratio_make() {
+  LegRatio r{};
+  for (int l = 1; l < SPH_LMAX; l++) r.c[l] = (double)(l - 1) / (double)l;
+  return r;
+}
+__constant__ LegRatio leg_ratio = leg_ratio_make();
 
 // Level sum of one accumulator column, sum_d c_d 2^(-7d), in one of three
 // exact forms (LS, chosen on the host from the bound on |c_d|):
@@ -248,6 +342,12 @@ __device__ __forceinline__ void tmem_wait4(uint32_t (&r)[S][4]) {
 #pragma unroll
   for (int d = 0; d < S; d++) asm volatile("" : "+r"(r[d][0]), "+r"(r[d][1]), "+r"(r[d][2]), "+r"(r[d][3]));
 }
+// a table load issued where it stands (volatile: not sunk below the stores)
+__device__ __forceinline__ double2 ld_table(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
 // bounded wait that also gives up once another role has raised the abort flag
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, const int* flag) {
   long long t0 = clock64();
@@ -255,6 +355,21 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, co
     if (*(volatile const int*)flag || clock64() - t0 > (1LL << 31)) return false;
   return true;
 }
+
+// Position in a ring of N slots: the slot and the parity of the current
+// round's completion (counters and divisions would cost the issuing warps
+// more than an MMA)
+template <int N>
+struct Ring {
+  int slot = 0;
+  uint32_t par = 0;
+  __device__ __forceinline__ void next() {
+    if (++slot == N) {
+      slot = 0;
+      par ^= 1;
+    }
+  }
+};
 
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... of the list.  The
 // stage ring and the two accumulator buffers run on counters that continue
@@ -268,16 +383,16 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
              double2* __restrict__ hs, int ld, double2* __restrict__ hsdiag, int* __restrict__ status,
              int never_wait) {
   using C = Cfg<S, KB>;
-  constexpr int N = C::N, IT = C::IT, STAGES = C::STAGES, HALF = C::IPT, EPI = C::EPI;
+  constexpr int N = C::N, IT = C::IT, STAGES = C::STAGES, IPT = C::IPT, EPI = C::EPI;
   constexpr int MMA_WARP = 4 * C::EG, TMA_WARP = 4 * C::EG + 1;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2], accbar, ebar, never;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform to the compiler
   const int L = P.ltop, nv = P.nv;
-  const int nit = L * nkb;  // pipeline iterations per tile
 
   if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -309,120 +424,121 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
   if (warp == TMA_WARP) {
     // ---- TMA producer: a full ring ahead of the MMAs ----
     if (lane == 0) {
-      long g = 0;  // iterations issued over all tiles
+      // a stage of the ring's first round is free, a later one once its last
+      // round's MMAs have completed (n: stages issued, up to a full ring)
+      Ring<STAGES> r;
+      int n = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
         const int2 tt = tiles[t];
         const int j0 = tt.x * 128, i0 = tt.y * IT;
-        for (int it = 0; it < nit; it++, g++) {
-          const int st = (int)(g % STAGES);
-          if (g >= STAGES) {  // the MMAs of g - STAGES have released the stage
-            const uint32_t par = (uint32_t)((g - STAGES) / STAGES) & 1;
-            long long t0 = clock64();
-            while (!mbar_try_wait(&empty[st], par)) {
-              if (*(volatile int*)&abort_flag || clock64() - t0 > (1LL << 31)) {
-                ok = false;
-                break;
-              }
+        for (int l = 0; l < L && ok; l++)
+          for (int kb = 0; kb < nkb; kb++) {
+            if (n == STAGES && !wait_or_abort(&empty[r.slot], r.par ^ 1, &abort_flag)) {
+              ok = false;
+              break;
             }
-            if (!ok) break;
+            uint8_t* a = smem + r.slot * C::STAGE;
+            mbar_expect_tx(&full[r.slot], C::STAGE);
+            tma_load_3d(a, &tmA, &full[r.slot], kb * KB, l * npA + j0, 0);
+            tma_load_3d(a + C::A_BYTES, &tmB, &full[r.slot], kb * KB, l * 4 * npB + 4 * i0, 0);
+            r.next();
+            if (n < STAGES) n++;
           }
-          const int l = it / nkb, kb = it % nkb;
-          uint8_t* a = smem + st * C::STAGE;
-          uint8_t* b = a + C::A_BYTES;
-          mbar_expect_tx(&full[st], C::STAGE);
-          tma_load_3d(a, &tmA, &full[st], kb * KB, l * npA + j0, 0);
-          tma_load_3d(b, &tmB, &full[st], kb * KB, l * 4 * npB + 4 * i0, 0);
-        }
       }
       if (!ok) atomicOr(status, L1G_STATUS_TIMEOUT);
       // the copies in flight land before the CTA's shared memory is released
       // (the MMA issuer may stop early; consumed stages return at once)
-      for (long q = g - STAGES > 0 ? g - STAGES : 0; q < g; q++)
-        mbar_wait(&full[q % STAGES], (uint32_t)(q / STAGES) & 1);
+      for (int q = 0; q < n; q++) {  // each stage's last round: this one below the position, else the one before
+        const int st = (r.slot + STAGES - 1 - q) % STAGES;
+        mbar_wait(&full[st], st < r.slot ? r.par : r.par ^ 1);
+      }
     }
     __syncwarp();
   } else if (warp == MMA_WARP) {
-    // ---- MMA issuer ----
-    if (lane == 0) {
-      long g = 0;   // pipeline iterations over all tiles
-      long gl = 0;  // accumulations (tile, l) over all tiles
+    // ---- MMA issuer: the whole warp walks the loop (uniform operands stay
+    // in uniform registers), one elected lane issues.  Issued from a branch
+    // of one lane instead, each MMA took about 110 clocks of that lane, more
+    // than its 77 clocks on the tensor core.
+    {
+      Ring<STAGES> r;
+      Ring<2> rt;     // accumulator buffers, one per l in turn
+      int fresh = 2;  // of them not yet used once
       bool ok = true;
+      // warp-uniform outcome
+      auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        return __all_sync(0xffffffffu, wait_or_abort(bar, parity, &abort_flag));
+      };
       if (never_wait) {
         // test hook: the consumer waits on a barrier that nothing arrives
         // at, with a short bound (about half a millisecond), and takes the
         // timeout path below (the other roles' waits keep their full bound)
         const long long t0 = clock64();
-        while (!mbar_try_wait(&never, 0))
-          if (clock64() - t0 > (1LL << 20)) {
-            ok = false;
-            break;
-          }
+        bool in_time = true;
+        while (in_time && !mbar_try_wait(&never, 0)) in_time = clock64() - t0 <= (1LL << 20);
+        ok = __all_sync(0xffffffffu, in_time);
       }
+      const uint64_t desc0 = desc_kblock<KB>(smem_u32(smem));
       for (int t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
-        for (int it = 0; it < nit; it++, g++) {
-          const int st = (int)(g % STAGES), kb = it % nkb, buf = (int)(gl & 1);
-          if (kb == 0 && gl >= 2 && !wait_or_abort(&tempty[buf], (uint32_t)((gl - 2) >> 1) & 1, &abort_flag)) {
-            ok = false;
-            break;
-          }
-          if (!wait_or_abort(&full[st], (uint32_t)(g / STAGES) & 1, &abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a0 = smem_u32(smem + st * C::STAGE);
-          const uint32_t b0 = a0 + C::A_BYTES;
-          // The S slices of B lie one after another in shared memory (one
-          // (S N)-row K-major tile) and the level accumulators N columns
-          // apart in TMEM, so A slice p times B slices 0..S-1-p is ONE MMA
-          // of width (S-p) N whose columns land on levels p..S-1.  The last
-          // block holds klast valid 32-byte steps (TMA zero-fills the rest;
-          // their MMAs are skipped).
-          const int nh = (kb == nkb - 1) ? klast : C::KSTEPS;
+        for (int l = 0; l < L && ok; l++) {
+          if (fresh > 0)
+            fresh--;
+          else
+            ok = wait(&tempty[rt.slot], rt.par ^ 1);
+          for (int kb = 0; kb < nkb && ok; kb++) {
+            ok = wait(&full[r.slot], r.par);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t ad0 = desc0 + (uint32_t)(r.slot * (C::STAGE >> 4)), bd0 = ad0 + (C::A_BYTES >> 4);
+            const uint32_t d0 = tmem + (uint32_t)(rt.slot * S * N);
+            // the last block holds klast valid 32-byte steps (TMA zero-fills
+            // the rest; their MMAs are skipped)
+            const int nh = (kb == nkb - 1) ? klast : C::KSTEPS;
+            if (elect_one()) {
+              // The S slices of B lie one after another in shared memory (one
+              // (S N)-row K-major tile) and the level accumulators N columns
+              // apart in TMEM, so A slice p times B slices 0..S-1-p is ONE MMA
+              // of width (S-p) N whose columns land on levels p..S-1
 #pragma unroll
-          for (int p = 0; p < S; p++)
+              for (int k = 0; k < C::KSTEPS; k++)
+                if (k < nh) {
 #pragma unroll
-            for (int h = 0; h < C::KSTEPS; h++) {
-              if (h >= nh) continue;
-              const uint64_t ad = desc_kblock<KB>(a0 + p * 128 * KB + h * 32);
-              const uint64_t bd = desc_kblock<KB>(b0 + h * 32);
-              const uint32_t acc = (kb > 0 || h > 0 || p > 0) ? 1u : 0u;
-              const uint32_t d = tmem + (uint32_t)(buf * S * N + p * N);
-              asm volatile(
-                  "{\n\t.reg .pred pa;\n\t"
-                  "setp.ne.b32 pa, %4, 0;\n\t"
-                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, pa;\n\t}" ::"r"(d),
-                  "l"(ad), "l"(bd), "r"(idesc_i8(128, (S - p) * N)), "r"(acc)
-                  : "memory");
+                  for (int p = 0; p < S; p++)
+                    mma_i8(d0 + p * N, ad0 + ((p * 128 * KB + k * 32) >> 4), bd0 + ((k * 32) >> 4),
+                           idesc_i8(128, (S - p) * N), (k > 0 || p > 0) ? 1u : (uint32_t)(kb > 0));
+                }
+              mma_commit(&empty[r.slot]);
+              if (kb == nkb - 1) mma_commit(&tfull[rt.slot]);
             }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_u32(&empty[st]))
-                       : "memory");
-          if (kb == nkb - 1) {
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&tfull[buf]))
-                         : "memory");
-            gl++;
+            __syncwarp();
+            r.next();
           }
+          rt.next();
         }
       }
-      if (!ok) {
-        atomicOr(status, L1G_STATUS_TIMEOUT);
-        *(volatile int*)&abort_flag = 1;
+      if (elect_one()) {
+        if (!ok) {
+          atomicOr(status, L1G_STATUS_TIMEOUT);
+          *(volatile int*)&abort_flag = 1;
+        }
+        mma_commit(&accbar);
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&accbar))
-                   : "memory");
     }
     __syncwarp();
   } else {
     // ---- epilogue warps ----
-    int16_t* sA = (int16_t*)(smem + STAGES * C::STAGE);  // [l][128]: eA - 12
+    double* sU = (double*)(smem + STAGES * C::STAGE);  // [IT][4]: k_I / |k_I| (0 for a zero row) and |k_I|
+    int* sK = (int*)(sU + 4 * IT);                   // [IT][4]: KZZ
+    int16_t* sA = (int16_t*)(sK + 4 * IT);            // [l][128]: eA - 12
     int16_t* sB = sA + SPH_LMAX * 128;                    // [l][IT][2]: eB
     const int g4 = warp & 3, hh = warp >> 2;
+    // Up to 5 slices the Legendre weights come from the polynomials, with x
+    // from the rows' unit vectors: the recursion's x and two last values per
+    // pair would take 6 registers each.  6 and 7 slices keep the recursion
+    // (its rounding is the reference's).
+    constexpr bool POLY = S <= 5;
     const uint32_t trow = tmem + ((uint32_t)(32 * g4) << 16);
-    long gl = 0;  // accumulations consumed over all tiles
+    Ring<2> rt;  // as the MMA issuer's
     bool ok = true;
     uint32_t ephase = 0;
     // barrier of the epilogue threads on an mbarrier, every wait bounded
@@ -438,8 +554,10 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
     // one tile ahead (behind the previous tile's interstitial part)
     constexpr int QA = (SPH_LMAX * 128 + EPI - 1) / EPI, QB = (SPH_LMAX * 2 * IT + EPI - 1) / EPI;
     int16_t pa[QA], pb[QB];
+    int2 tn = make_int2(0, 0);          // the next tile
     auto fetch = [&](int t) {  // volatile loads: issued here, ahead of their use
-      const int j0 = split::ld_early(&tiles[t].x) * 128, i0 = split::ld_early(&tiles[t].y) * IT;
+      tn = make_int2(split::ld_early(&tiles[t].x), split::ld_early(&tiles[t].y));
+      const int j0 = tn.x * 128, i0 = tn.y * IT;
 #pragma unroll
       for (int k = 0; k < QA; k++) {
         const int q = tid + k * EPI, l = q >> 7, J = j0 + (q & 127);
@@ -455,9 +573,27 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
     };
     if (blockIdx.x < ntile) fetch(blockIdx.x);
     for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-      const int2 tt = tiles[t];
-      const int j0 = tt.x * 128, i0 = tt.y * IT;
-      // scale tables of this tile for every l, written once the previous
+      const int j0 = tn.x * 128, i0 = tn.y * IT;
+      // this thread's J row, and one I row per thread of the first warps
+      const int J = j0 + 32 * g4 + lane;
+      const bool jin = J < nv;
+      const int Jr = min(J, nv - 1), Ir = min(i0 + tid, nv - 1);
+      const double rj = P.rk[Jr], vj = rj > 0.0 ? 1.0 / rj : 0.0;
+      const double ux = P.xk[Jr] * vj, uy = P.yk[Jr] * vj, uz = P.zk[Jr] * vj;
+      const int k1 = P.kzz[3 * Jr], k2 = P.kzz[3 * Jr + 1], k3 = P.kzz[3 * Jr + 2];
+      double ri = 0.0, xi = 0.0, yi = 0.0, zi = 0.0;
+      int ki1 = 0, ki2 = 0, ki3 = 0;
+      if (tid < IT) {
+        ri = P.rk[Ir];
+        const double vi = ri > 0.0 ? 1.0 / ri : 0.0;
+        xi = P.xk[Ir] * vi;
+        yi = P.yk[Ir] * vi;
+        zi = P.zk[Ir] * vi;
+        ki1 = P.kzz[3 * Ir];
+        ki2 = P.kzz[3 * Ir + 1];
+        ki3 = P.kzz[3 * Ir + 2];
+      }
+      // row and scale tables of this tile, written once the previous
       // tile's readers are past the first barrier
       if (!epi_sync()) {
         ok = false;
@@ -469,34 +605,92 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
 #pragma unroll
       for (int k = 0; k < QB; k++)
         if (tid + k * EPI < L * 2 * IT) sB[tid + k * EPI] = pb[k];
+      if (tid < IT) {
+        sU[4 * tid] = xi;
+        sU[4 * tid + 1] = yi;
+        sU[4 * tid + 2] = zi;
+        sU[4 * tid + 3] = ri;
+        sK[4 * tid] = ki1;
+        sK[4 * tid + 1] = ki2;
+        sK[4 * tid + 2] = ki3;
+      }
       if (!epi_sync()) {
         ok = false;
         break;
       }
-      const int J = j0 + 32 * g4 + lane;
-      const bool jin = J < nv;
-      const double xj = jin ? P.xk[J] : 0.0, yj = jin ? P.yk[J] : 0.0, zj = jin ? P.zk[J] : 0.0;
-      const double rj = jin ? P.rk[J] : 0.0;
-      double x[HALF], pm1[HALF], pm2[HALF];
-      double2 aS[HALF], aH[HALF];
+      // cosine of the pair's k vectors (li: I within the tile)
+      auto cosine = [&](int li) { return fma(ux, sU[4 * li], fma(uy, sU[4 * li + 1], uz * sU[4 * li + 2])); };
+      double x[POLY ? 1 : IPT], pm1[POLY ? 1 : IPT], pm2[POLY ? 1 : IPT];
+      double2 aS[IPT], aH[IPT];
+      unsigned top = 0, flat = 0;  // pairs along one line (hamilt.F's UTOP branch); pairs with a (nearly) zero row
 #pragma unroll
-      for (int u = 0; u < HALF; u++) {
-        const int I = i0 + hh * HALF + u;
+      for (int u = 0; u < IPT; u++) {
+        const int li = hh * IPT + u;
         double xx = 0.0;
-        if (jin && I < nv) {
-          xx = P.xk[I] * xj + P.yk[I] * yj + P.zk[I] * zj;
-          const double den = P.rk[I] * rj;
-          if (den > 1.0e-8) xx = xx / den;
+        if (jin && i0 + li < nv) {
+          xx = cosine(li);
+          const double den = rj * sU[4 * li + 3];
+          if (!(den > 1.0e-8)) {  // the reference's x is k_J.k_I itself: at most 1e-8
+            flat |= 1u << u;
+            xx *= den;
+          }
         }
-        x[u] = xx;
-        pm1[u] = xx;   // P_1
-        pm2[u] = 1.0;  // P_0
+        if (!(fabs(xx) < 0.9999999)) top |= 1u << u;
+        if (!POLY) {
+          x[u] = xx;
+          pm1[u] = xx;   // P_1
+          pm2[u] = 1.0;  // P_0
+        }
         aS[u] = aH[u] = make_double2(0.0, 0.0);
       }
-      for (int l = 0; l < L; l++, gl++) {
-        const int buf = (int)(gl & 1);
+      for (int l = 0; l < L; l++, rt.next()) {
+        const int buf = rt.slot;
+        // scales (2l+1) P_l 2^(eA + eB) of this thread's pairs: formed
+        // before the wait, which hides them when the MMAs are behind
+        const int ea = sA[l * 128 + 32 * g4 + lane] + (LS == 2 ? -7 * (S - 1) : 0);
+        double sS[IPT], sH[IPT];
+        {
+          double w[IPT];
+          if (POLY) {
+            double xx[IPT];
+#pragma unroll
+            for (int u = 0; u < IPT; u++) {
+              xx[u] = cosine(hh * IPT + u);
+              if ((flat >> u) & 1) xx[u] = 0.0;
+            }
+            leg_weights(l, xx, top, w);
+          } else {
+            // Legendre recursion (hamilt.F:250-281, UTOP branch)
+            const double cl = leg_ratio.c[l], fl = (double)(2 * l + 1);
+#pragma unroll
+            for (int u = 0; u < IPT; u++) {
+              double pl;
+              if (l == 0)
+                pl = 1.0;
+              else if (l == 1)
+                pl = x[u];
+              else {
+                if (!((top >> u) & 1)) {
+                  const double pplx = x[u] * pm1[u];
+                  pl = pplx + cl * (pplx - pm2[u]);
+                } else {
+                  pl = x[u] * pm1[u];
+                }
+                pm2[u] = pm1[u];
+                pm1[u] = pl;
+              }
+              w[u] = fl * pl;
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < IPT; u++) {
+            const short2 sb = *reinterpret_cast<const short2*>(sB + (l * IT + hh * IPT + u) * 2);
+            sS[u] = w[u] * pow2i(ea + sb.x);
+            sH[u] = w[u] * pow2i(ea + sb.y);
+          }
+        }
         // warp-uniform outcome: the TMEM loads below are .sync.aligned
-        if (!__all_sync(0xffffffffu, wait_or_abort(&tfull[buf], (uint32_t)(gl >> 1) & 1, &abort_flag))) {
+        if (!__all_sync(0xffffffffu, wait_or_abort(&tfull[buf], rt.par, &abort_flag))) {
           ok = false;
           if (lane == 0) atomicOr(status, L1G_STATUS_TIMEOUT);
           break;
@@ -506,17 +700,15 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
           break;
         }
         tc_fence_after();
-        const int ea = sA[l * 128 + 32 * g4 + lane] + (LS == 2 ? -7 * (S - 1) : 0);
-        const double cl = (l >= 2) ? (double)(l - 1) / (double)l : 0.0, fl = (double)(2 * l + 1);
-        // 4 real columns per I: S re, S im, H re, H im; this thread's HALF I
-        // start at column 4 HALF hh; one I (4 columns x S levels) per load
-        const uint32_t tcol = trow + (uint32_t)(buf * S * N + 4 * HALF * hh);
+        // 4 real columns per I: S re, S im, H re, H im; this thread's I start
+        // at column 4 IPT hh; one I (4 columns x S levels) per load
+        const uint32_t tcol = trow + (uint32_t)(buf * S * N + 4 * IPT * hh);
 #pragma unroll
-        for (int u = 0; u < HALF; u++) {
+        for (int u = 0; u < IPT; u++) {
           uint32_t r[S][4];
           tmem_ld4<S>(r, tcol + 4 * u, N);
           tmem_wait4<S>(r);
-          if (u == HALF - 1) {
+          if (u == IPT - 1) {
             // all columns of this buffer read: hand it back to the MMA issuer
             tc_fence_before();
             __syncwarp();
@@ -531,29 +723,10 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
             for (int d = 0; d < S; d++) rr[d] = r[d][m];
             v[m] = level_sum<S, LS>(rr);
           }
-          // Legendre weight (hamilt.F:250-281 recursion, UTOP branch)
-          double pl;
-          if (l == 0)
-            pl = 1.0;
-          else if (l == 1)
-            pl = x[u];
-          else {
-            if (fabs(x[u]) < 0.9999999) {
-              const double pplx = x[u] * pm1[u];
-              pl = pplx + cl * (pplx - pm2[u]);
-            } else {
-              pl = x[u] * pm1[u];
-            }
-            pm2[u] = pm1[u];
-            pm1[u] = pl;
-          }
-          const double wl = fl * pl;
-          const int16_t* sb = sB + (l * IT + hh * HALF + u) * 2;
-          const double sS = wl * pow2i(ea + sb[0]), sH = wl * pow2i(ea + sb[1]);
-          aS[u].x = fma(v[0], sS, aS[u].x);
-          aS[u].y = fma(v[1], sS, aS[u].y);
-          aH[u].x = fma(v[2], sH, aH[u].x);
-          aH[u].y = fma(v[3], sH, aH[u].y);
+          aS[u].x = fma(v[0], sS[u], aS[u].x);
+          aS[u].y = fma(v[1], sS[u], aS[u].y);
+          aH[u].x = fma(v[2], sH[u], aH[u].x);
+          aH[u].y = fma(v[3], sH[u], aH[u].y);
         }
       }
       if (!ok) {
@@ -561,39 +734,44 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
         break;
       }
       if (t + (int)gridDim.x < ntile) fetch(t + gridDim.x);
-      // interstitial + write (hamilt.F:289-345, 459-466, calkpt.F:164): every
-      // load of the HALF pairs first (the HS stores might alias them), then
-      // the stores; I past NV reads a valid row and stores nothing
+      // interstitial + write (hamilt.F:289-345, 459-466, calkpt.F:164)
       if (jin) {
         const int nx = 2 * T.d1 + 1, ny = 2 * T.d2 + 1;
-        const int k1 = P.kzz[3 * J], k2 = P.kzz[3 * J + 1], k3 = P.kzz[3 * J + 2];
-        double2 th[HALF], wp[HALF];
-        double x2[HALF];
+        // table values of NG pairs at a time, the next NG in flight while
+        // these are written; I past NV reads a valid entry and stores nothing
+        constexpr int NG = 2;
+        double2 th[2][NG], wp[2][NG];
+        auto gather = [&](int g, double2(&a)[NG], double2(&b)[NG]) {
 #pragma unroll
-        for (int u = 0; u < HALF; u++) {
-          const int I = min(i0 + hh * HALF + u, nv - 1);
-          x2[u] = xj * P.xk[I] + yj * P.yk[I] + zj * P.zk[I];
-          const int d1 = k1 - P.kzz[3 * I] + T.d1, d2 = k2 - P.kzz[3 * I + 1] + T.d2,
-                    d3 = k3 - P.kzz[3 * I + 2] + T.d3;
-          const size_t ci = ((size_t)d3 * ny + d2) * nx + d1;
-          th[u] = tab[2 * ci];
-          wp[u] = tab[2 * ci + 1];
-        }
-        bool bad = false;  // a written element is not finite
-#pragma unroll
-        for (int u = 0; u < HALF; u++) {
-          const int I = i0 + hh * HALF + u;
-          if (I >= nv || J > I) continue;
-          const double2 s = cadd(th[u], aS[u]);
-          const double2 h = cadd(cadd(cscale(th[u], x2[u]), wp[u]), aH[u]);
-          if (J == I) {
-            hs[(size_t)I * ld + I] = h;
-            hsdiag[I] = s;
-          } else {
-            hs[(size_t)I * ld + J] = s;  // S upper: HS(J,I)
-            hs[(size_t)J * ld + I] = h;  // H lower: HS(I,J)
+          for (int w = 0; w < NG; w++) {
+            const int li = hh * IPT + g * NG + w;
+            const int d1 = k1 - sK[4 * li] + T.d1, d2 = k2 - sK[4 * li + 1] + T.d2, d3 = k3 - sK[4 * li + 2] + T.d3;
+            const size_t ci = ((size_t)d3 * ny + d2) * nx + d1;
+            a[w] = ld_table(tab + 2 * ci);
+            b[w] = ld_table(tab + 2 * ci + 1);
           }
-          bad |= l1g_nonfinite(s) | l1g_nonfinite(h);
+        };
+        bool bad = false;  // a written element is not finite
+        gather(0, th[0], wp[0]);
+#pragma unroll
+        for (int g = 0; g < IPT / NG; g++) {
+          if (g + 1 < IPT / NG) gather(g + 1, th[(g + 1) & 1], wp[(g + 1) & 1]);
+#pragma unroll
+          for (int w = 0; w < NG; w++) {
+            const int u = g * NG + w, li = hh * IPT + u, I = i0 + li;
+            if (I >= nv || J > I) continue;
+            const double x2 = cosine(li) * (rj * sU[4 * li + 3]);
+            const double2 s = cadd(th[g & 1][w], aS[u]);
+            const double2 hv = cadd(cadd(cscale(th[g & 1][w], x2), wp[g & 1][w]), aH[u]);
+            if (J == I) {
+              hs[(size_t)I * ld + I] = hv;
+              hsdiag[I] = s;
+            } else {
+              hs[(size_t)I * ld + J] = s;   // S upper: HS(J,I)
+              hs[(size_t)J * ld + I] = hv;  // H lower: HS(I,J)
+            }
+            bad |= l1g_nonfinite(s) | l1g_nonfinite(hv);
+          }
         }
         if (bad) atomicOr(status, L1G_STATUS_NONFINITE);
       }

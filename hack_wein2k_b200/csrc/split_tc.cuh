@@ -131,6 +131,30 @@ template <int KB>
 __device__ __forceinline__ uint64_t desc_kblock(uint32_t saddr) {
   return KB == 128 ? desc_sw128(saddr) : desc_sw64(saddr);
 }
+// one lane of a converged warp (the same one every time)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+// one MMA (issued by one lane): D[d] (+)= A B, acc = 0 overwrites D
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred pa;\n\t"
+      "setp.ne.b32 pa, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, pa;\n\t}" ::"r"(d),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+      : "memory");
+}
+// an arrival on bar once every MMA issued so far by this lane has completed
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
+}
 // instruction descriptor: D s32, A s8, B s8, both K-major, M x N
 __host__ __device__ constexpr uint32_t idesc_i8(int M, int N) {
   return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
