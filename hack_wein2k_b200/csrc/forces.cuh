@@ -779,16 +779,15 @@ __global__ void __launch_bounds__(256) k_force_trans(const double2* __restrict__
   }
 }
 
-// Cf = f c, Ce = f eps c per band (cj: their conjugates, for the split
-// path's products C conj(Cf)^T, which take no conjugate themselves)
+// conj(f c) and conj(f eps c) per band, for the products C X^T, which take
+// no conjugate themselves
 __global__ void k_force_weight(int n, int nb, const double2* __restrict__ C, int ldc, const double* __restrict__ f,
-                               const double* __restrict__ eps, int cj, double2* __restrict__ Cf,
+                               const double* __restrict__ eps, double2* __restrict__ Cf,
                                double2* __restrict__ Ce) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (i >= n) return;
-  double2 v = C[(size_t)b * ldc + i];
-  if (cj) v = cconj(v);
+  const double2 v = cconj(C[(size_t)b * ldc + i]);
   Cf[(size_t)b * n + i] = cscale(v, f[b]);
   Ce[(size_t)b * n + i] = cscale(v, f[b] * eps[b]);
 }

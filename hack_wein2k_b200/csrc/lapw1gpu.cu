@@ -5,8 +5,8 @@
 //   HAMILT  -> k_albl, k_phase, k_table, k_sph_coef, k_spherical, k_lo
 //   ZSWAP   -> folded into the HAMILT writes (diag(HS) = H, HSDIAG = S)
 //   HNS     -> k_hns_alm, k_hns_tmul, k_hns_lo_ops (operands), then
-//              k_hns_gemm + library ZGEMM panels (FP64) or the
-//              split-precision tcgen05 path, and k_hns_lo
+//              k_tri_gemm (FP64, DMMA) or the split-precision tcgen05 path,
+//              each with its LO-LO block
 //   HORB    -> k_horb_rows, k_horb_pairs per U-atom and l
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
@@ -113,7 +113,7 @@ struct lapw1gpu_context {
   cublasHandle_t blas[L1G_MAX_SETS] = {};  // library ZGEMMs, one handle (and workspace) per scratch set
   cusolverDnHandle_t solver = nullptr;      // the eigen-solve (lapw1gpu_seclr4)
   // tunables (lapw1gpu_autotune)
-  int hns_diag_b = 512;    // FP64 HNS: diagonal block of the blocked ZHER2M form
+  int hns_diag_b = 512;    // kept for callers that set it; the FP64 HNS update is one product without blocks
   int split_group = 16;    // split HNS: row tiles per rasterisation group
   int sph_tc = 1;          // split precision: spherical part on tcgen05 (1) or FP64 (0)
   int sph_kb = 128;        // k_sph_tc: bytes of K per pipeline stage (64: deep ring, 128: two stages)
@@ -852,46 +852,34 @@ static int launch_hns_ops(lapw1gpu_context* c, const DevProb& P, const double2* 
   return l1g_launch_status(__FILE__, __LINE__);
 }
 
-// The FP64 HNS update in the blocked form of ZHER2M (zher2m.f:69-80):
-// diagonal blocks of B rows run in k_hns_gemm (64-row tiles, lower triangle
-// only), the rows below each diagonal block in one library ZGEMM per block
-// column.  B is a tunable (lapw1gpu_autotune), 512 by default.
-static const int2* tiles_hns_diag(lapw1gpu_kpoint* k, int n, int B, int* count) {
-  return kp_tiles(k, "hnsdiag:" + std::to_string(n) + ":" + std::to_string(B), count, [&](std::vector<int2>& t) {
-    const int per = B / HNS_T;
-    const int nt = (n + HNS_T - 1) / HNS_T;
-    for (int b0 = 0; b0 < nt; b0 += per)
-      for (int bi = b0; bi < std::min(nt, b0 + per); bi++)
-        for (int bj = b0; bj <= bi; bj++) t.push_back(make_int2(bi, bj));
-  });
-}
-
-// (hp: after the panels of each column group, its event; groups whose
-// columns reach the LO block are left for the caller to record)
-static int hns_panels_zgemm(cublasHandle_t h, int n, int nv, int npad, int K, int B, const double2* Lop,
-                            const double2* Rop, double2* hs, int ld, cudaStream_t s, HnsPipe* hp) {
-  if (!h) return LAPW1GPU_ERR_CUDA;
-  const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0);
-  if (hp && hp->groups > 0 && !hp->fixed) {  // groups of whole panels
-    const int np = (n + B - 1) / B, G = std::min(hp->groups, np);
-    hp->groups = G;
-    for (int g = 0; g <= G; g++) hp->col[g] = std::min(n, (int)((long)np * g / G) * B);
-  }
-  int g = 0;
-  for (int c0 = 0; c0 < n; c0 += B) {
-    const int w = std::min(B, n - c0);
-    const int r0 = c0 + w, m = n - r0;
-    // HS(r0:n, c0:c0+w) += L(r0:n, :) R(c0:c0+w, :)^T ; L, R column-major npad x K
-    if (m > 0 && cublasZgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, m, w, K, &one, (const cuDoubleComplex*)(Lop + r0), npad,
-                             (const cuDoubleComplex*)(Rop + c0), npad, &one,
-                             (cuDoubleComplex*)(hs + (size_t)c0 * ld + r0), ld) != CUBLAS_STATUS_SUCCESS)
-      return LAPW1GPU_ERR_CUDA;
-    if (hp && g < hp->groups && r0 >= hp->col[g + 1]) {
-      if (hp->col[g + 1] <= nv && cudaEventRecord(hp->ev[g], s) == cudaSuccess) hp->recorded[g] = true;
-      g++;
-    }
-  }
-  return LAPW1GPU_OK;
+// Lower-triangle FP64 product (k_tri_gemm) over the tile columns [c0, c1) of
+// out, c0 a multiple of TRI_COLS (c1 too unless it is n); c (the context)
+// may be null.  64 x 64 tiles, 32 x 32 while the 64-wide ones would leave
+// SMs without a block.
+#define TRI_COLS 64
+static int launch_tri(lapw1gpu_context* c, int n, int c0, int c1, int K, const double2* L, int ldl, const double2* R,
+                      int ldr, double2* out, int ld, int ovw, int* status, cudaStream_t s, int* nl) {
+  const int nsm = c ? c->nsm : 148;
+  const long n64 = (n + 63) / 64;
+  const bool wide = n64 * (n64 + 1) / 2 >= 2 * nsm;
+  const int T = wide ? 64 : 32, nb = (n + T - 1) / T;
+  const void* fn = wide ? (const void*)k_tri_gemm<32> : (const void*)k_tri_gemm<16>;
+  const int bytes = tri_smem_bytes(T / 2);
+  if (c ? !c->smem(fn, bytes)
+        : cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+    return LAPW1GPU_ERR_CUDA;
+  auto first = [&](int col) {  // tiles left of column block col
+    const long b = std::min(nb, (col + T - 1) / T);
+    return b * nb - b * (b - 1) / 2;
+  };
+  const long t0 = first(c0), t1 = first(c1);
+  if (t1 <= t0) return LAPW1GPU_OK;
+  if (wide)
+    k_tri_gemm<32><<<(unsigned)(t1 - t0), TRI_THREADS, bytes, s>>>(n, K, nb, t0, L, ldl, R, ldr, out, ld, ovw, status);
+  else
+    k_tri_gemm<16><<<(unsigned)(t1 - t0), TRI_THREADS, bytes, s>>>(n, K, nb, t0, L, ldl, R, ldr, out, ld, ovw, status);
+  ++*nl;
+  return l1g_launch_status(__FILE__, __LINE__);
 }
 
 }  // extern "C"
@@ -1181,33 +1169,33 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     } else {
       rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, s, &nl);
       if (rc) return rc;
-      int ntiles = 0;
-      const int2* tl = tiles_hns_diag(k, n, c->hns_diag_b, &ntiles);
-      if (!tl) return LAPW1GPU_ERR_NOMEM;
-      nl++;
       if (ev) CK(cudaEventRecord(ev[14], s));
-      k_hns_gemm<<<ntiles, 256, 0, s>>>(n, k->npad, K, tl, Lop, Rop, d_hs, ldhs);
-      rc = hns_panels_zgemm(c->handle(set, s), n, nv, k->npad, K, c->hns_diag_b, Lop, Rop, d_hs, ldhs, s, hp);
+      // column group by column group (groups whose columns reach the LO block
+      // are recorded after it)
+      const int G = hp && hp->groups > 0 ? hp->groups : 1;
+      for (int g = 0; g < G && !rc; g++) {
+        rc = launch_tri(c, n, G > 1 ? hp->col[g] : 0, G > 1 ? hp->col[g + 1] : n, K, Lop, k->npad, Rop, k->npad, d_hs,
+                        ldhs, 0, nullptr, s, &nl);
+        if (G > 1 && !rc && hp->col[g + 1] <= nv) {
+          CK(cudaEventRecord(hp->ev[g], s));
+          hp->recorded[g] = true;
+        }
+      }
       if (ev && !rc) CK(cudaEventRecord(ev[15], s));
     }
     if (rc) return rc;
     if (k->nlo > 0) {
-      nl++;
-      // T = C2 CLM^T (nlo x nlo, K = NDF 25): in split precision from the
-      // auxiliary stream's tensor-core product, else by library ZGEMM; its
-      // lower triangle into HS
-      double2* T = (double2*)c->sbuf(set, "hnsLoT", sizeof(double2) * (size_t)k->nlo * k->nlo);
-      if (!T) return LAPW1GPU_ERR_NOMEM;
-      if (!hns_fork) {
-        cublasHandle_t h = c->handle(set, s);
-        if (!h) return LAPW1GPU_ERR_NOMEM;
-        const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0), zero = make_cuDoubleComplex(0.0, 0.0);
-        if (cublasZgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, k->nlo, k->nlo, ndf * nsl2, &one, (const cuDoubleComplex*)C2lo,
-                        k->nlo, (const cuDoubleComplex*)Clo, k->nlo, &zero, (cuDoubleComplex*)T,
-                        k->nlo) != CUBLAS_STATUS_SUCCESS)
-          return LAPW1GPU_ERR_CUDA;
+      // C2 CLM^T on the LO block: FP64 added in place; in split precision
+      // the auxiliary stream's tensor-core product, its lower triangle into HS
+      if (hns_fork) {
+        double2* T = (double2*)c->sbuf(set, "hnsLoT", sizeof(double2) * (size_t)k->nlo * k->nlo);
+        if (!T) return LAPW1GPU_ERR_NOMEM;
+        nl++;
+        k_add_lower<<<dim3((k->nlo + 127) / 128, k->nlo), 128, 0, s>>>(nv, k->nlo, T, d_hs, ldhs, c->d_status);
+      } else if (int rc2 = launch_tri(c, k->nlo, 0, k->nlo, ndf * nsl2, C2lo, k->nlo, Clo, k->nlo,
+                                      d_hs + (size_t)nv * ldhs + nv, ldhs, 0, nullptr, s, &nl)) {
+        return rc2;
       }
-      k_add_lower<<<dim3((k->nlo + 127) / 128, k->nlo), 128, 0, s>>>(nv, k->nlo, T, d_hs, ldhs, c->d_status);
     }
     CK(cudaGetLastError());
     if (hp)  // the groups whose columns reach the LO block end here
@@ -1418,7 +1406,7 @@ int lapw1gpu_get_tuning(lapw1gpu_context* c, lapw1gpu_tuning* t) {
 
 int lapw1gpu_set_tuning(lapw1gpu_context* c, const lapw1gpu_tuning* t) {
   if (!c || !t) return LAPW1GPU_ERR_ARG;
-  if (t->hns_diag_b < HNS_T || t->hns_diag_b % HNS_T || t->split_group < 1 || t->batch_sets < 1 ||
+  if (t->hns_diag_b < TRI_COLS || t->hns_diag_b % TRI_COLS || t->split_group < 1 || t->batch_sets < 1 ||
       t->batch_sets > L1G_MAX_SETS || (t->sph_tc != 0 && t->sph_tc != 1) ||
       (t->sph_kblock != 64 && t->sph_kblock != 128))
     return LAPW1GPU_ERR_RANGE;
@@ -1469,9 +1457,7 @@ int lapw1gpu_autotune(lapw1gpu_context* c, lapw1gpu_kpoint* kp, double* d_hs, in
     return LAPW1GPU_OK;
   };
   int rc = LAPW1GPU_OK;
-  if (c->prec == LAPW1GPU_PREC_FP64) {
-    rc = tune(&c->hns_diag_b, {256, 512, 1024, 2048}, T_TOTAL);
-  } else {
+  if (c->prec == LAPW1GPU_PREC_SPLIT) {
     if (sph_tc_supported(c->slices)) rc = tune(&c->sph_tc, {1, 0}, T_TOTAL);
     // the K block (and with it the ring depth) of k_sph_tc: 128-byte blocks
     // exist up to 5 slices
@@ -1506,7 +1492,7 @@ static int sph_granule(const lapw1gpu_context* c) {
   return SPH_T;
 }
 static int hns_granule(const lapw1gpu_context* c) {
-  if (c->prec != LAPW1GPU_PREC_SPLIT) return c->hns_diag_b;
+  if (c->prec != LAPW1GPU_PREC_SPLIT) return TRI_COLS;
   switch (c->slices_hns) {
     case 2: return split::Cfg<2>::JT;
     case 3: return split::Cfg<3>::JT;
@@ -1565,7 +1551,7 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
   HnsPipe hp;
   const bool pipe = overlap && (stages & 2) && !k->nohns && !((stages & 4) && !k->orbs.empty());
   if (pipe) {
-    // about 8 groups of columns, boundaries on a multiple of both tile widths
+    // up to 8 groups of about 512 columns or more, boundaries on a multiple of both tile widths
     const int a = sph_granule(c), b = hns_granule(c);
     int gcd = a, r = b;
     while (r) {
@@ -1576,8 +1562,11 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
     const long gran = (long)a / gcd * b;
     int G = 0;
     hp.col[0] = 0;
-    for (int g = 1; g < 8; g++) {
-      const int cb = (int)(((long)n * g / 8) / gran * gran);
+    // (at N = 704 eight groups made the launches three times as long as one,
+    // for copies of 0.14 ms in all)
+    const int ng = std::max(1, std::min(8, n / 512));
+    for (int g = 1; g < ng; g++) {
+      const int cb = (int)(((long)n * g / ng) / gran * gran);
       if (cb > hp.col[G] && cb < n) hp.col[++G] = cb;
     }
     hp.col[++G] = n;
@@ -1825,16 +1814,16 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
   k_phase<<<dim3((k->npad + 127) / 128, ndf), 128, 0, s>>>(P);
   k_sph_coef<<<nat, 32, 0, s>>>(P, coef);
   const bool split_rho = c->prec == LAPW1GPU_PREC_SPLIT;
-  k_force_weight<<<dim3((n + 127) / 128, nb), 128, 0, s>>>(n, nb, C, ldc, d_occ, d_eps, split_rho ? 1 : 0, Cf, Ce);
+  k_force_weight<<<dim3((n + 127) / 128, nb), 128, 0, s>>>(n, nb, C, ldc, d_occ, d_eps, Cf, Ce);
   nlf += 4;  // k_albl, k_phase, k_sph_coef, k_force_weight
   CK(cudaGetLastError());
-  // rho(J,I) = sum_b f_b c_b(J) conj(c_b(I)), column-major n x n, and rhoE:
-  // Hermitian, and only J < I is read.  FP64: the library forms the upper
-  // triangle alone (half the flops of a full product).  Split precision:
-  // the int8 slice-product kernel of the HNS update forms the lower
-  // triangle of C X^T with X = conj(Cf) (k_force_weight conjugated it), i.e.
-  // conj(rho(J,I)) at (I, J) (rt = 1 below).
-  int rt = 0;
+  // rho(J,I) = sum_b f_b c_b(J) conj(c_b(I)) and rhoE: Hermitian, and only
+  // J < I is read.  Both precisions form the lower triangle of C X^T with
+  // X = conj(Cf) (k_force_weight conjugated it), i.e. conj(rho(J,I)) at (I, J)
+  // of a column-major n x n block, written, not added (no zero fill: every
+  // lower-triangle element the force kernels read is a product tile's
+  // element): by k_tri_gemm, or by the int8 slice products of the HNS update.
+  const int rt = 1;
   if (split_rho) {
     const double2* Cn = C;
     if (ldc != n) {  // the operand kernels take one row stride for both sides
@@ -1844,23 +1833,16 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
                            cudaMemcpyDeviceToDevice, s));
       Cn = Cc;
     }
-    // written, not added (no zero fill): every lower-triangle element the
-    // force kernels read is a product tile's element
     int nlr = 0;
     int rc = split_hns_gemm(c, k, 0, n, n, nb, Cn, Cf, rho, n, c->slices_frc, s, &nlr, nullptr, nullptr, 0, 3, 1);
     if (!rc)
       rc = split_hns_gemm(c, k, 0, n, n, nb, Cn, Ce, rhoe, n, c->slices_frc, s, &nlr, nullptr, nullptr, 0, 3, 1);
     if (rc) return rc;
     nlf += nlr;
-    rt = 1;
   } else {
-    const double rzero = 0.0;
-    if (cublasZherkx(h, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, n, nb, &one, (const cuDoubleComplex*)Cf, n,
-                     (const cuDoubleComplex*)C, ldc, &rzero, (cuDoubleComplex*)rho, n) != CUBLAS_STATUS_SUCCESS ||
-        cublasZherkx(h, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, n, nb, &one, (const cuDoubleComplex*)Ce, n,
-                     (const cuDoubleComplex*)C, ldc, &rzero, (cuDoubleComplex*)rhoe, n) != CUBLAS_STATUS_SUCCESS)
-      return LAPW1GPU_ERR_CUDA;
-    nlf += 2;
+    int rc = launch_tri(c, n, 0, n, nb, C, ldc, Cf, n, rho, n, 1, nullptr, s, &nlf);
+    if (!rc) rc = launch_tri(c, n, 0, n, nb, C, ldc, Ce, n, rhoe, n, 1, nullptr, s, &nlf);
+    if (rc) return rc;
   }
   if (timed) CK(cudaEventRecord(c->fev[1], s));
   // G c (k_force_gscale) and, in split precision, its k-major copy (G c)^T:
@@ -2205,9 +2187,9 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[L1G_NOALLOC_BYT
 static void* g_noalloc_addr[L1G_NOALLOC_MAXDEV];  // device address of the array, per device
 
 // bookkeeping tables of one problem, built on the device (one thread):
-// atom type / first atom per type, the LOHNS ranges, the triangle tiles
-__global__ void k_noalloc_tables(int nat, const int* __restrict__ mult, const int* __restrict__ ilo, int ntri,
-                                 int* atype, int* afirst, LoRange* lor, int2* tiles) {
+// atom type / first atom per type, the LOHNS ranges
+__global__ void k_noalloc_tables(int nat, const int* __restrict__ mult, const int* __restrict__ ilo, int* atype,
+                                 int* afirst, LoRange* lor) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   for (int a = 0, q = 0; a < nat; a++) {
     afirst[a] = q;
@@ -2221,8 +2203,6 @@ __global__ void k_noalloc_tables(int nat, const int* __restrict__ mult, const in
         nnlo = r.i2;
         lor[nr++] = r;
       }
-  for (int bi = 0, t = 0; bi < ntri; bi++)
-    for (int bj = 0; bj <= bi; bj++) tiles[t++] = make_int2(bi, bj);
 }
 
 // true when SPHBES would refuse an argument RMT |k+G| of this problem's
@@ -2268,8 +2248,6 @@ extern "C" int lapw1gpu_hns_noalloc(const lapw1gpu_problem* p, double* d_hs_, in
   int nlor = 0;
   for (int jn = 0; jn < nat; jn++)
     for (int l = 0; l <= L1G_LOMAX; l++) nlor += p->ilo[jn * L4 + l];
-  const int ntri = (n + HNS_T - 1) / HNS_T;
-  const int ntiles = ntri * (ntri + 1) / 2;
 
   // carve the array: inputs first, then the intermediates; the input copies
   // are issued as the regions are taken (no host-side bookkeeping storage)
@@ -2339,7 +2317,6 @@ extern "C" int lapw1gpu_hns_noalloc(const lapw1gpu_problem* p, double* d_hs_, in
   P.dplo = (const double*)in(p->dplo, sizeof(double) * nat * L4);
   const double2* d_tns = (const double2*)in(p->tns, sizeof(double2) * nat * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2);
   LoRange* d_lor = (LoRange*)take(sizeof(LoRange) * (nlor > 0 ? nlor : 1));
-  int2* d_tiles = (int2*)take(sizeof(int2) * ntiles);
   P.al = (double*)take(sizeof(double) * (size_t)nat * ltop * nvpad);
   P.bl = (double*)take(sizeof(double) * (size_t)nat * ltop * nvpad);
   P.phase = (double2*)take(sizeof(double2) * (size_t)ndf * npad);
@@ -2357,15 +2334,17 @@ extern "C" int lapw1gpu_hns_noalloc(const lapw1gpu_problem* p, double* d_hs_, in
       CK(cudaMemcpyAsync(pend[q].dst, pend[q].src, pend[q].bytes, cudaMemcpyHostToDevice, s));
   // the array keeps the previous call's contents: the status word must start at 0
   CK(cudaMemsetAsync(d_status, 0, sizeof(int), s));
-  k_noalloc_tables<<<1, 32, 0, s>>>(nat, P.mult, P.ilo, ntri, d_atype, d_afirst, d_lor, d_tiles);
+  k_noalloc_tables<<<1, 32, 0, s>>>(nat, P.mult, P.ilo, d_atype, d_afirst, d_lor);
   k_albl<<<dim3((nvpad + 127) / 128, nat), 128, 0, s>>>(P, d_status);
   k_phase<<<dim3((npad + 127) / 128, ndf), 128, 0, s>>>(P);
   int nops = 0;
   rc = launch_hns_ops(nullptr, P, d_tns, d_lor, nlor, Lop, Rop, Clo, C2lo, s, &nops);
   if (rc) return rc;
-  k_hns_gemm<<<(unsigned)ntiles, 256, 0, s>>>(n, npad, K, d_tiles, Lop, Rop, d_hs, ldhs);
-  if (p->nlo > 0)
-    k_hns_lo<<<dim3((p->nlo + 127) / 128, p->nlo), 128, 0, s>>>(nv, p->nlo, ndf * nsl2, C2lo, Clo, d_hs, ldhs);
+  rc = launch_tri(nullptr, n, 0, n, K, Lop, npad, Rop, npad, d_hs, ldhs, 0, nullptr, s, &nops);
+  if (!rc && p->nlo > 0)
+    rc = launch_tri(nullptr, p->nlo, 0, p->nlo, ndf * nsl2, C2lo, p->nlo, Clo, p->nlo, d_hs + (size_t)nv * ldhs + nv, ldhs,
+                    0, nullptr, s, &nops);
+  if (rc) return rc;
   // a non-finite element of the updated HS sets L1G_STATUS_NONFINITE, as
   // the HNS stage of the allocating entry points reports it
   if (d_status_out) k_check_finite<<<1184, 256, 0, s>>>(n, d_hs, ldhs, nullptr, d_status);
