@@ -42,60 +42,14 @@
 
 #define FRC_2PI 6.283185307179586476925287
 
-// Rows of the spherical force operands, per (type, l, row): the J side
-// (a, b) and the I side, S = vif (a, chn b) and H = vif (mAA a + mAB b,
-// mBA a + mBB b), so that each l term of a pair is one 2-vector dot
-// product per side.  Rows nv..nvpad-1 are zero (k_albl zeroes them).
-__global__ void k_force_rows(DevProb P, const SphCoef* __restrict__ coef, double2* __restrict__ rowJ,
-                             double2* __restrict__ rowI) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x, tl = blockIdx.y;  // tl = type * ltop + l
-  if (r >= P.nvpad) return;
-  const size_t o = (size_t)tl * P.nvpad + r;
-  const double a = P.al[o], b = P.bl[o];
-  const SphCoef c = coef[tl];
-  rowJ[o] = cmk(a, b);
-  rowI[2 * o] = cmk(c.vif * a, c.vif * (c.chn * b));
-  rowI[2 * o + 1] = cmk(c.vif * (c.mAA * a + c.mAB * b), c.vif * (c.mBA * a + c.mBB * b));
-}
-
 #define FRC_THREADS 256
-#define FRC_MAXA 16  // equivalent atoms per staged chunk (a type with more reads its phases from global)
-#define FRC_LT 11    // l count of the specialised kernel (lmax = 10)
-
-// types per staged chunk: as many as the shared memory holds twice
-__host__ __device__ constexpr int frc_tc(int lt) { return lt <= FRC_LT ? 5 : 4; }
-
-__device__ __forceinline__ void frc_cp16(void* dst, const void* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void frc_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void frc_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// A chunk of types from t0: up to TC types whose equivalent atoms fit
-// FRC_MAXA; a single type with more atoms forms a chunk of its own whose
-// phases are not staged.
-struct FrcChunk {
-  int ntc, na, staged;
-};
-template <int TC>
-__device__ __forceinline__ FrcChunk frc_chunk(const DevProb& P, int t0) {
-  FrcChunk c{0, 0, 1};
-  while (c.ntc < TC && t0 + c.ntc < P.nat && c.na + P.mult[t0 + c.ntc] <= FRC_MAXA) c.na += P.mult[t0 + c.ntc++];
-  if (c.ntc == 0) c = FrcChunk{1, 0, 0};
-  return c;
-}
-
 // dynamic shared memory: two stages of type rows (J: 1, I: 2 double2 per
 // row and l) and of phases, two buffers of the per-warp force totals of a
 // chunk's atoms (one per warp and component), and -4 pi KZZ of the tile's
 // 64 rows
 #define FRC_WARPS (FRC_THREADS / 32)
 __host__ __device__ constexpr int frc_smem_bytes(int lt) {
-  return (2 * frc_tc(lt) * lt * SPH_T * 3 + 2 * 2 * FRC_MAXA * SPH_T) * 16 + 2 * FRC_MAXA * 3 * FRC_WARPS * 8 +
+  return (2 * pr_tc(lt) * lt * SPH_T * 3 + 2 * 2 * PR_MAXA * SPH_T) * 16 + 2 * PR_MAXA * 3 * FRC_WARPS * 8 +
          2 * SPH_T * 4 * 8;
 }
 
@@ -106,7 +60,7 @@ __host__ __device__ constexpr int frc_smem_bytes(int lt) {
 // shared-memory reads (about one cycle each: the addresses of a read are
 // 8 or 4 distinct 16-byte words) stay below the FP64 pipe's rate.  The
 // Legendre weights, rho, rhoE and dK of the four pairs stay in registers
-// for all types.  The type rows (k_force_rows) and the phases of a chunk
+// for all types.  The type rows (k_pair_rows) and the phases of a chunk
 // are copied into shared memory by cp.async one chunk ahead (double
 // buffer), one warp per 32-row segment.  One block barrier per chunk: the
 // per-warp force totals of a chunk go to one of two buffers and are summed
@@ -116,13 +70,13 @@ __global__ void __launch_bounds__(FRC_THREADS, 1)
     k_force_sph(DevProb P, const int2* __restrict__ tiles, const double2* __restrict__ rowJ,
                 const double2* __restrict__ rowI, TabDesc T, const double2* __restrict__ rho,
                 const double2* __restrict__ rhoe, int ldr, int rt, double* __restrict__ F, double* __restrict__ bins) {
-  constexpr int TC = frc_tc(LT);
+  constexpr int TC = pr_tc(LT);
   extern __shared__ double2 sm2[];
   double2* sJ = sm2;                       // [2][TC][LT][SPH_T]
   double2* sI = sJ + 2 * TC * LT * SPH_T;  // [2][TC][LT][SPH_T][S, H]
-  double2* sP = sI + 4 * TC * LT * SPH_T;  // [2][J, I][FRC_MAXA][SPH_T]
-  double* red = reinterpret_cast<double*>(sP + 4 * FRC_MAXA * SPH_T);  // [2][FRC_MAXA][3][warps]
-  double* sK = red + 2 * FRC_MAXA * 3 * FRC_WARPS;                       // [J 0..31, I 32..63][4]
+  double2* sP = sI + 4 * TC * LT * SPH_T;  // [2][J, I][PR_MAXA][SPH_T]
+  double* red = reinterpret_cast<double*>(sP + 4 * PR_MAXA * SPH_T);  // [2][PR_MAXA][3][warps]
+  double* sK = red + 2 * PR_MAXA * 3 * FRC_WARPS;                       // [J 0..31, I 32..63][4]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int2 t = tiles[blockIdx.x];
   const int i0 = t.x * SPH_T, j0 = t.y * SPH_T;
@@ -132,31 +86,31 @@ __global__ void __launch_bounds__(FRC_THREADS, 1)
   // (type, l) rows of consecutive types are consecutive in rowJ / rowI:
   // the chunk's rows are k = 0 .. ntc ltop - 1 from row t0 ltop, and with
   // ltop = LT also consecutive in shared memory
-  auto stage = [&](int st, int t0, const FrcChunk& ch) {
+  auto stage = [&](int st, int t0, const PairChunk& ch) {
     double2* dJ = sJ + st * TC * LT * SPH_T;
     double2* dI = sI + st * 2 * TC * LT * SPH_T;
     const size_t g0 = (size_t)t0 * ltop;
     for (int k = warp; k < ch.ntc * ltop; k += FRC_THREADS / 32) {
       const int ks = GUARD ? (k / ltop) * LT + k % ltop : k;
       const double2* src = rowJ + (g0 + k) * nvpad + j0;
-      frc_cp16(dJ + ks * SPH_T + lane, src + lane);
+      pr_cp16(dJ + ks * SPH_T + lane, src + lane);
       const double2* srci = rowI + 2 * ((g0 + k) * nvpad + i0);
-      frc_cp16(dI + ks * 2 * SPH_T + lane, srci + lane);
-      frc_cp16(dI + ks * 2 * SPH_T + SPH_T + lane, srci + SPH_T + lane);
+      pr_cp16(dI + ks * 2 * SPH_T + lane, srci + lane);
+      pr_cp16(dI + ks * 2 * SPH_T + SPH_T + lane, srci + SPH_T + lane);
     }
     if (ch.staged) {
-      double2* dP = sP + st * 2 * FRC_MAXA * SPH_T;
+      double2* dP = sP + st * 2 * PR_MAXA * SPH_T;
       const int a0c = P.afirst[t0];
       for (int k = warp; k < ch.na * 2; k += FRC_THREADS / 32) {
         const int side = k & 1, e = k >> 1;
-        frc_cp16(dP + (side * FRC_MAXA + e) * SPH_T + lane,
+        pr_cp16(dP + (side * PR_MAXA + e) * SPH_T + lane,
                  P.phase + (size_t)(a0c + e) * P.npad + (side ? i0 : j0) + lane);
       }
     }
-    frc_commit();
+    pr_commit();
   };
 
-  FrcChunk ch = frc_chunk<TC>(P, 0);
+  PairChunk ch = pr_chunk<TC>(P, 0);
   stage(0, 0, ch);
   // the pair term carries -2 (2 pi dK) = -4 pi (KZZ_I - KZZ_J): per row
   // -4 pi KZZ, read once per atom
@@ -215,7 +169,7 @@ __global__ void __launch_bounds__(FRC_THREADS, 1)
   // one thread per (atom, component)
   auto flush = [&](int rb, int a0, int na) {
     if (tid < na * 3) {
-      const double* r = red + ((size_t)rb * FRC_MAXA * 3 + tid) * FRC_WARPS;
+      const double* r = red + ((size_t)rb * PR_MAXA * 3 + tid) * FRC_WARPS;
       double sacc = 0.0;
 #pragma unroll
       for (int w = 0; w < FRC_WARPS; w++) sacc += r[w];
@@ -226,18 +180,18 @@ __global__ void __launch_bounds__(FRC_THREADS, 1)
   int pa0 = 0, pna = 0;  // atoms of the previous chunk, flushed after this chunk's barrier
   for (int t0 = 0; t0 < nat;) {
     const int t1 = t0 + ch.ntc;
-    frc_wait<0>();    // this thread's copies of the chunk (issued one chunk earlier)
+    pr_wait<0>();    // this thread's copies of the chunk (issued one chunk earlier)
     __syncthreads();  // every thread's copies landed; every warp is past the previous chunk
-    FrcChunk nx{0, 0, 1};
+    PairChunk nx{0, 0, 1};
     if (t1 < nat) {  // into the stage the previous chunk read
-      nx = frc_chunk<TC>(P, t1);
+      nx = pr_chunk<TC>(P, t1);
       stage(st ^ 1, t1, nx);
     }
     flush(st ^ 1, pa0, pna);
     const double2* cJ = sJ + st * TC * LT * SPH_T;
     const double2* cI = sI + st * 2 * TC * LT * SPH_T;
-    const double2* cPJ = sP + st * 2 * FRC_MAXA * SPH_T;
-    const double2* cPI = cPJ + FRC_MAXA * SPH_T;
+    const double2* cPJ = sP + st * 2 * PR_MAXA * SPH_T;
+    const double2* cPI = cPJ + PR_MAXA * SPH_T;
     const int a0c = P.afirst[t0];
     // l sums of type tc for the four pairs
     auto lsum = [&](int tc, double(&tS)[4], double(&tH)[4]) {
@@ -316,7 +270,7 @@ __global__ void __launch_bounds__(FRC_THREADS, 1)
       const int b = e * SPH_T;
       const double2 fj[2] = {cPJ[b + jl0], cPJ[b + jl0 + 8]}, fi[2] = {cPI[b + il0], cPI[b + il0 + 4]};
       const double v = fterm(fj, fi, tS, tH);
-      if ((lane & 7) == 0 && lane < 24) red[(((size_t)st * FRC_MAXA + e) * 3 + (lane >> 3)) * FRC_WARPS + warp] = v;
+      if ((lane & 7) == 0 && lane < 24) red[(((size_t)st * PR_MAXA + e) * 3 + (lane >> 3)) * FRC_WARPS + warp] = v;
     };
     if (ch.staged && ch.na == ch.ntc) {
       // one atom per type (slot tc): the force terms of type tc - 1 are
@@ -823,20 +777,20 @@ __global__ void __launch_bounds__(256, 1) k_force_hns_z(int zc, int nsl2, int K,
   // wave of work after it)
   for (int i = tid; i < nb * nsl2 * nsl2; i += blockDim.x) {
     const int blk = i / (nsl2 * nsl2), r = i % (nsl2 * nsl2), lm = r / nsl2, b = r % nsl2;
-    frc_cp16(&sT[(blk * L1G_NSL2 + lm) * L1G_NSL2 + b], &T[((size_t)(b0 + blk) * L1G_NSL2 + lm) * L1G_NSL2 + b]);
+    pr_cp16(&sT[(blk * L1G_NSL2 + lm) * L1G_NSL2 + b], &T[((size_t)(b0 + blk) * L1G_NSL2 + lm) * L1G_NSL2 + b]);
   }
   for (int i = tid; i < nc * 3 * nsl2; i += blockDim.x) {
     const int cl = i / (3 * nsl2), r = i % (3 * nsl2), part = r / nsl2, b = r % nsl2;
     double2* dst = &sY[(cl * 3 + part) * L1G_NSL2 + b];
     if (part < 2)
-      frc_cp16(dst, &Y[(size_t)(c0 + cl) * K + (size_t)a * 2 * nsl2 + part * nsl2 + b]);
+      pr_cp16(dst, &Y[(size_t)(c0 + cl) * K + (size_t)a * 2 * nsl2 + part * nsl2 + b]);
     else if (Yc)
-      frc_cp16(dst, &Yc[(size_t)(c0 + cl) * Kc + (size_t)a * nsl2 + b]);
+      pr_cp16(dst, &Yc[(size_t)(c0 + cl) * Kc + (size_t)a * nsl2 + b]);
     else
       *dst = cmk(0.0, 0.0);
   }
-  frc_commit();
-  frc_wait<0>();
+  pr_commit();
+  pr_wait<0>();
   __syncthreads();
   // warp w: columns 32 (w % 4) + lane, outputs: zc = 0 the row r = w / 4
   // (lm = 0 .. nsl2-1), zc = 1 the lm half w / 4 of the single row

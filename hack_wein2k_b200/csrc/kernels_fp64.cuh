@@ -196,21 +196,15 @@ __global__ void k_table(DevProb P, TabDesc T, const double2* warp, double2* tab)
 // This kernel keeps that loop order: the Legendre weights w_l = (2l+1) P_l
 // of each pair are computed once with the reference's recursion (UTOP
 // branch included, hamilt.F:250-281) and held in registers; per atom type
-// the J-side {AL, BL} and the I-side VIF {AL, CHN BL, hA, hB} are staged in
-// shared memory; PHASE is formed as sum_eq phi_a(J) conj(phi_a(I)) from the
-// per-row phases.  That is 6 FMA per (pair, type, l) plus the phase
-// products, instead of 16 for the same sum as a GEMM over explicit (l, r).
-// Thread (tj, ti) owns rows J = j0 + tj + 16u and columns I = i0 + ti + 16v
-// (u, v in {0,1}), so shared-memory reads are conflict-free.
+// the J-side {AL, BL} and the I-side VIF {AL, CHN BL, hA, hB} rows
+// (k_pair_rows) are staged in shared memory; PHASE is formed as
+// sum_eq phi_a(J) conj(phi_a(I)) from the per-row phases.  That is 6 FP64
+// operations per (pair, type, l) plus the phase products, instead of 16 for
+// the same sum as a GEMM over explicit (l, r).
 // ---------------------------------------------------------------------
 #define SPH_T 32
-#define SPH_TC 8
 #define SPH_THREADS 256
 #define SPH_LMAX 13
-#define SPH_MAXA 32  // equivalent atoms whose phases one chunk stages
-// dynamic shared memory: per staged type 1 J-side and 2 I-side double2 per
-// (l, row), plus the J and I phases of up to SPH_MAXA atoms
-#define SPH_DYN_SMEM ((3 * SPH_TC * SPH_LMAX * SPH_T + 2 * SPH_MAXA * SPH_T) * 16)
 
 struct SphCoef {  // per (type, l)
   double vif, chn, mAA, mAB, mBA, mBB;
@@ -234,155 +228,199 @@ __global__ void k_sph_coef(DevProb P, SphCoef* coef) {
   coef[jn * P.ltop + l] = c;
 }
 
+// Operand rows of the pair kernels (k_spherical, k_force_sph), per (type, l, row): the J side
+// (a, b) and the I side, S = vif (a, chn b) and H = vif (mAA a + mAB b,
+// mBA a + mBB b), so that each l term of a pair is one 2-vector dot
+// product per side.  Rows nv..nvpad-1 are zero (k_albl zeroes them).
+__global__ void k_pair_rows(DevProb P, const SphCoef* __restrict__ coef, double2* __restrict__ rowJ,
+                             double2* __restrict__ rowI) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x, tl = blockIdx.y;  // tl = type * ltop + l
+  if (r >= P.nvpad) return;
+  const size_t o = (size_t)tl * P.nvpad + r;
+  const double a = P.al[o], b = P.bl[o];
+  const SphCoef c = coef[tl];
+  rowJ[o] = cmk(a, b);
+  rowI[2 * o] = cmk(c.vif * a, c.vif * (c.chn * b));
+  rowI[2 * o + 1] = cmk(c.vif * (c.mAA * a + c.mAB * b), c.vif * (c.mBA * a + c.mBB * b));
+}
+
+#define PR_MAXA 16  // equivalent atoms per staged chunk (a type with more reads its phases from global)
+#define PR_LT 11    // l count of the specialised kernel (lmax = 10)
+
+// types per staged chunk: as many as the shared memory holds twice
+__host__ __device__ constexpr int pr_tc(int lt) { return lt <= PR_LT ? 5 : 4; }
+
+__device__ __forceinline__ void pr_cp16(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void pr_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void pr_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// A chunk of types from t0: up to TC types whose equivalent atoms fit
+// PR_MAXA; a single type with more atoms forms a chunk of its own whose
+// phases are not staged.
+struct PairChunk {
+  int ntc, na, staged;
+};
+template <int TC>
+__device__ __forceinline__ PairChunk pr_chunk(const DevProb& P, int t0) {
+  PairChunk c{0, 0, 1};
+  while (c.ntc < TC && t0 + c.ntc < P.nat && c.na + P.mult[t0 + c.ntc] <= PR_MAXA) c.na += P.mult[t0 + c.ntc++];
+  if (c.ntc == 0) c = PairChunk{1, 0, 0};
+  return c;
+}
+
+// dynamic shared memory of k_spherical: two stages of type rows (J: 1, I: 2
+// double2 per row and l) and of phases
+__host__ __device__ constexpr int sph_smem_bytes(int lt) {
+  return (2 * pr_tc(lt) * lt * SPH_T * 3 + 2 * 2 * PR_MAXA * SPH_T) * 16;
+}
+
+// One block per 32 x 32 pair tile, 256 threads, bound by the FP64 pipe's
+// issue.  Thread (warp, lane) owns the 2 x 2 pairs J = j0 + jl0 + {0, 8},
+// I = i0 + il0 + {0, 4} with jl0 = 16 (warp & 1) + (lane & 7), il0 =
+// 8 (warp >> 1) + (lane >> 3): a warp reads 8 distinct J rows and 4 distinct
+// I rows per l, 6 shared loads for 24 FP64 operations, each about one cycle
+// (8 or fewer distinct words).  The chunk of types after the current one is
+// copied by cp.async meanwhile (one block barrier per chunk), and for
+// one-atom types the phase products of a type are formed beside the l sums
+// of the next.  LT: l values (unrolled); GUARD: ltop may be below LT.
+template <int LT, bool GUARD>
 __global__ void __launch_bounds__(SPH_THREADS, 1)
-    k_spherical(DevProb P, const int2* __restrict__ tiles, const SphCoef* __restrict__ coef,
-                const double2* __restrict__ tab, TabDesc T, double2* __restrict__ hs, int ld,
-                double2* __restrict__ hsdiag) {
+    k_spherical(DevProb P, const int2* __restrict__ tiles, const double2* __restrict__ rowJ,
+                const double2* __restrict__ rowI, const double2* __restrict__ tab, TabDesc T, double2* __restrict__ hs,
+                int ld, double2* __restrict__ hsdiag) {
+  constexpr int TC = pr_tc(LT);
   extern __shared__ double2 sm2[];
-  // staged per type chunk: J side (AL, BL) [tc][l][32], I side VIF-scaled
-  // (AL, CHN BL) and (hA, hB) [tc][l][32][2], phases [atom][32] for J and I
-  double2* sJ = sm2;
-  double2* sI = sJ + SPH_TC * SPH_LMAX * SPH_T;
-  double2* sPJ = sI + 2 * SPH_TC * SPH_LMAX * SPH_T;
-  double2* sPI = sPJ + SPH_MAXA * SPH_T;
-  const int tid = threadIdx.x;
-  const int tj = tid & 15, ti = tid >> 4;
+  double2* sJ = sm2;                       // [2][TC][LT][SPH_T]
+  double2* sI = sJ + 2 * TC * LT * SPH_T;  // [2][TC][LT][SPH_T][S, H]
+  double2* sP = sI + 4 * TC * LT * SPH_T;  // [2][J, I][PR_MAXA][SPH_T]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int2 t = tiles[blockIdx.x];
   const int i0 = t.x * SPH_T, j0 = t.y * SPH_T;
-  const int nv = P.nv, ltop = P.ltop, nat = P.nat;
+  const int nv = P.nv, ltop = P.ltop, nat = P.nat, nvpad = P.nvpad;
+  const int jl0 = (warp & 1) * 16 + (lane & 7), il0 = (warp >> 1) * 8 + (lane >> 3);
 
-  // Legendre weights (2l+1) P_l(x_JI) of the four owned pairs
-  double w[4][SPH_LMAX];
-#pragma unroll
-  for (int u = 0; u < 2; u++)
-#pragma unroll
-    for (int v = 0; v < 2; v++) {
-      const int q = u * 2 + v;
-      const int J = j0 + tj + 16 * u, I = i0 + ti + 16 * v;
-      double x = 0.0;
-      if (J < nv && I < nv) {
-        x = P.xk[I] * P.xk[J] + P.yk[I] * P.yk[J] + P.zk[I] * P.zk[J];
-        double den = P.rk[I] * P.rk[J];
-        if (den > 1.0e-8) x = x / den;
-      }
-      const bool top = !(fabs(x) < 0.9999999);
-      double pm2 = 1.0, pm1 = x;
-      w[q][0] = 1.0;
-      w[q][1] = 3.0 * x;
-#pragma unroll
-      for (int l = 2; l < SPH_LMAX; l++) {
-        double pl;
-        if (!top) {
-          const double pplx = x * pm1;
-          const double pply = pplx - pm2;
-          pl = pplx + ((double)(l - 1) / (double)l) * pply;
-        } else {
-          pl = x * pm1;
-        }
-        pm2 = pm1;
-        pm1 = pl;
-        w[q][l] = (double)(2 * l + 1) * pl;
+  // (type, l) rows of consecutive types are consecutive in rowJ / rowI
+  auto stage = [&](int st, int t0, const PairChunk& ch) {
+    double2* dJ = sJ + st * TC * LT * SPH_T;
+    double2* dI = sI + st * 2 * TC * LT * SPH_T;
+    const size_t g0 = (size_t)t0 * ltop;
+    for (int k = warp; k < ch.ntc * ltop; k += SPH_THREADS / 32) {
+      const int ks = GUARD ? (k / ltop) * LT + k % ltop : k;
+      const double2* src = rowJ + (g0 + k) * nvpad + j0;
+      pr_cp16(dJ + ks * SPH_T + lane, src + lane);
+      const double2* srci = rowI + 2 * ((g0 + k) * nvpad + i0);
+      pr_cp16(dI + ks * 2 * SPH_T + lane, srci + lane);
+      pr_cp16(dI + ks * 2 * SPH_T + SPH_T + lane, srci + SPH_T + lane);
+    }
+    if (ch.staged) {
+      double2* dP = sP + st * 2 * PR_MAXA * SPH_T;
+      const int a0c = P.afirst[t0];
+      for (int k = warp; k < ch.na * 2; k += SPH_THREADS / 32) {
+        const int side = k & 1, e = k >> 1;
+        pr_cp16(dP + (side * PR_MAXA + e) * SPH_T + lane,
+                P.phase + (size_t)(a0c + e) * P.npad + (side ? i0 : j0) + lane);
       }
     }
+    pr_commit();
+  };
+  PairChunk ch = pr_chunk<TC>(P, 0);
+  stage(0, 0, ch);
 
+  // Legendre weights (2l+1) P_l(x_JI) of the four owned pairs
+  double w[4][LT];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int J = j0 + jl0 + 8 * (q >> 1), I = i0 + il0 + 4 * (q & 1);
+    double x = 0.0;
+    if (J < nv && I < nv) {
+      x = P.xk[I] * P.xk[J] + P.yk[I] * P.yk[J] + P.zk[I] * P.zk[J];
+      const double den = P.rk[I] * P.rk[J];
+      if (den > 1.0e-8) x = x / den;
+    }
+    const bool top = !(fabs(x) < 0.9999999);
+    double pm2 = 1.0, pm1 = x;
+    w[q][0] = 1.0;
+    if (LT > 1) w[q][1] = 3.0 * x;
+#pragma unroll
+    for (int l = 2; l < LT; l++) {
+      double pl;
+      if (!top) {
+        const double pplx = x * pm1;
+        pl = pplx + ((double)(l - 1) / (double)l) * (pplx - pm2);
+      } else {
+        pl = x * pm1;
+      }
+      pm2 = pm1;
+      pm1 = pl;
+      w[q][l] = (double)(2 * l + 1) * pl;
+    }
+  }
   double2 aS[4], aH[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) aS[q] = aH[q] = cmk(0.0, 0.0);
 
+  int st = 0;
   for (int t0 = 0; t0 < nat;) {
-    // chunk of types whose equivalent atoms fit the staged phase rows
-    int ntc = 0, na = 0;
-    while (ntc < SPH_TC && t0 + ntc < nat && na + P.mult[t0 + ntc] <= SPH_MAXA) na += P.mult[t0 + ntc++];
-    const bool staged = ntc > 0;
-    if (!staged) ntc = 1;  // one type with more atoms than SPH_MAXA: phases from global memory
-    const int a0c = P.afirst[t0];
-    __syncthreads();
-    for (int idx = tid; idx < ntc * ltop * SPH_T; idx += SPH_THREADS) {
-      const int r = idx % SPH_T, l = (idx / SPH_T) % ltop, tc = idx / (SPH_T * ltop);
-      const int jn = t0 + tc;
-      const size_t ob = ((size_t)jn * ltop + l) * P.nvpad;
-      const int J = j0 + r, I = i0 + r;
-      double aj = 0.0, bj = 0.0, ai = 0.0, bi = 0.0;
-      if (J < nv) {
-        aj = P.al[ob + J];
-        bj = P.bl[ob + J];
-      }
-      if (I < nv) {
-        ai = P.al[ob + I];
-        bi = P.bl[ob + I];
-      }
-      const SphCoef c = coef[jn * ltop + l];
-      const int s = (tc * SPH_LMAX + l) * SPH_T + r;
-      sJ[s] = cmk(aj, bj);
-      sI[2 * s] = cmk(c.vif * ai, c.vif * (c.chn * bi));
-      sI[2 * s + 1] = cmk(c.vif * (c.mAA * ai + c.mAB * bi), c.vif * (c.mBA * ai + c.mBB * bi));
+    const int t1 = t0 + ch.ntc;
+    pr_wait<0>();
+    __syncthreads();  // every thread's copies landed; every warp is past the previous chunk
+    PairChunk nx{0, 0, 1};
+    if (t1 < nat) {  // into the stage the previous chunk read
+      nx = pr_chunk<TC>(P, t1);
+      stage(st ^ 1, t1, nx);
     }
-    if (staged)
-      for (int idx = tid; idx < na * SPH_T; idx += SPH_THREADS) {
-        const int r = idx % SPH_T, e = idx / SPH_T;
-        const double2* pa = P.phase + (size_t)(a0c + e) * P.npad;
-        sPJ[idx] = pa[j0 + r];
-        sPI[idx] = pa[i0 + r];
-      }
-    __syncthreads();
-    for (int tc = 0; tc < ntc; tc++) {
-      const int jn = t0 + tc;
-      double tS[4], tH[4];
+    const double2* cJ = sJ + st * TC * LT * SPH_T + jl0;
+    const double2* cI = sI + st * 2 * TC * LT * SPH_T + 2 * il0;
+    const double2* cPJ = sP + st * 2 * PR_MAXA * SPH_T + jl0;
+    const double2* cPI = sP + st * 2 * PR_MAXA * SPH_T + PR_MAXA * SPH_T + il0;
+    // l sums of type tc for the four pairs (the row values of l + 1 are read
+    // while l is summed)
+    auto lsum = [&](int tc, double(&tS)[4], double(&tH)[4]) {
+      const double2* bJ = cJ + tc * LT * SPH_T;
+      const double2* bI = cI + tc * LT * 2 * SPH_T;
+      double2 av[2] = {bJ[0], bJ[8]}, sv[2] = {bI[0], bI[8]}, hv[2] = {bI[1], bI[9]};
 #pragma unroll
-      for (int q = 0; q < 4; q++) tS[q] = tH[q] = 0.0;
-#pragma unroll
-      for (int l = 0; l < SPH_LMAX; l++) {
-        if (l < ltop) {
-          const int s = (tc * SPH_LMAX + l) * SPH_T;
-          double2 jv[2], is[2], ih[2];
-#pragma unroll
-          for (int u = 0; u < 2; u++) jv[u] = sJ[s + tj + 16 * u];
-#pragma unroll
-          for (int v = 0; v < 2; v++) {
-            is[v] = sI[2 * (s + ti + 16 * v)];
-            ih[v] = sI[2 * (s + ti + 16 * v) + 1];
-          }
-#pragma unroll
-          for (int u = 0; u < 2; u++)
-#pragma unroll
-            for (int v = 0; v < 2; v++) {
-              const int q = u * 2 + v;
-              const double sv = fma(jv[u].y, is[v].y, jv[u].x * is[v].x);
-              const double hv = fma(jv[u].y, ih[v].y, jv[u].x * ih[v].x);
-              tS[q] = fma(w[q][l], sv, tS[q]);
-              tH[q] = fma(w[q][l], hv, tH[q]);
-            }
-        }
-      }
-      // PHASE = sum over the equivalent atoms of this type
-      double2 ph[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) ph[q] = cmk(0.0, 0.0);
-      const int ae = P.afirst[jn], me = P.mult[jn];
-      for (int e = 0; e < me; e++) {
-        double2 fj[2], fi[2];
-        if (staged) {
-          const int b = (ae - a0c + e) * SPH_T;
-#pragma unroll
-          for (int u = 0; u < 2; u++) fj[u] = sPJ[b + tj + 16 * u];
-#pragma unroll
-          for (int v = 0; v < 2; v++) fi[v] = sPI[b + ti + 16 * v];
-        } else {
-          const double2* pa = P.phase + (size_t)(ae + e) * P.npad;
-#pragma unroll
-          for (int u = 0; u < 2; u++) fj[u] = pa[j0 + tj + 16 * u];
-#pragma unroll
-          for (int v = 0; v < 2; v++) fi[v] = pa[i0 + ti + 16 * v];
+      for (int l = 0; l < LT; l++) {
+        if (GUARD && l >= ltop) break;
+        const double2 a0 = av[0], a1 = av[1], s0 = sv[0], s1 = sv[1], h0 = hv[0], h1 = hv[1];
+        if (l + 1 < LT) {
+          const int o = (l + 1) * SPH_T;
+          av[0] = bJ[o];
+          av[1] = bJ[o + 8];
+          sv[0] = bI[2 * o];
+          sv[1] = bI[2 * o + 8];
+          hv[0] = bI[2 * o + 1];
+          hv[1] = bI[2 * o + 9];
         }
 #pragma unroll
-        for (int u = 0; u < 2; u++)
-#pragma unroll
-          for (int v = 0; v < 2; v++) {
-            const int q = u * 2 + v;
-            ph[q].x = fma(fj[u].x, fi[v].x, fma(fj[u].y, fi[v].y, ph[q].x));
-            ph[q].y = fma(fj[u].y, fi[v].x, fma(-fj[u].x, fi[v].y, ph[q].y));
+        for (int q = 0; q < 4; q++) {
+          const double2 a = (q >> 1) ? a1 : a0, s = (q & 1) ? s1 : s0, h = (q & 1) ? h1 : h0;
+          if (l == 0) {  // w_0 = P_0 = 1
+            tS[q] = fma(a.y, s.y, a.x * s.x);
+            tH[q] = fma(a.y, h.y, a.x * h.x);
+          } else {
+            tS[q] = fma(w[q][l], fma(a.y, s.y, a.x * s.x), tS[q]);
+            tH[q] = fma(w[q][l], fma(a.y, h.y, a.x * h.x), tH[q]);
           }
+        }
       }
+    };
+    // phi_J conj(phi_I) of one atom added to ph
+    auto phase = [&](const double2(&fj)[2], const double2(&fi)[2], double2(&ph)[4]) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const double2 a = fj[q >> 1], b = fi[q & 1];
+        ph[q].x = fma(a.x, b.x, fma(a.y, b.y, ph[q].x));
+        ph[q].y = fma(a.y, b.x, fma(-a.x, b.y, ph[q].y));
+      }
+    };
+    auto add = [&](const double2(&ph)[4], const double(&tS)[4], const double(&tH)[4]) {
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         aS[q].x = fma(ph[q].x, tS[q], aS[q].x);
@@ -390,20 +428,69 @@ __global__ void __launch_bounds__(SPH_THREADS, 1)
         aH[q].x = fma(ph[q].x, tH[q], aH[q].x);
         aH[q].y = fma(ph[q].y, tH[q], aH[q].y);
       }
+    };
+    auto one = [&](int e, const double(&tS)[4], const double(&tH)[4]) {  // a one-atom type, staged slot e
+      const double2 fj[2] = {cPJ[e * SPH_T], cPJ[e * SPH_T + 8]}, fi[2] = {cPI[e * SPH_T], cPI[e * SPH_T + 4]};
+      double2 ph[4] = {};
+      phase(fj, fi, ph);
+      add(ph, tS, tH);
+    };
+    if (ch.staged && ch.na == ch.ntc) {
+      double pS[4], pH[4];
+      lsum(0, pS, pH);
+      for (int tc = 1; tc < ch.ntc; tc++) {
+        double tS[4], tH[4];
+        lsum(tc, tS, tH);
+        one(tc - 1, pS, pH);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          pS[q] = tS[q];
+          pH[q] = tH[q];
+        }
+      }
+      one(ch.ntc - 1, pS, pH);
+    } else {
+      const int a0c = P.afirst[t0];
+      for (int tc = 0; tc < ch.ntc; tc++) {
+        double tS[4], tH[4];
+        lsum(tc, tS, tH);
+        const int jn = t0 + tc, ae = P.afirst[jn], me = P.mult[jn];
+        double2 ph[4] = {};
+        for (int e = 0; e < me; e++) {
+          double2 fj[2], fi[2];
+          if (ch.staged) {
+            const int b = (ae - a0c + e) * SPH_T;
+            fj[0] = cPJ[b];
+            fj[1] = cPJ[b + 8];
+            fi[0] = cPI[b];
+            fi[1] = cPI[b + 4];
+          } else {  // a type with more atoms than a chunk stages
+            const double2* pa = P.phase + (size_t)(ae + e) * P.npad;
+            fj[0] = pa[j0 + jl0];
+            fj[1] = pa[j0 + jl0 + 8];
+            fi[0] = pa[i0 + il0];
+            fi[1] = pa[i0 + il0 + 4];
+          }
+          phase(fj, fi, ph);
+        }
+        add(ph, tS, tH);
+      }
     }
-    t0 += ntc;
+    t0 = t1;
+    ch = nx;
+    st ^= 1;
   }
   // interstitial + write (hamilt.F:289-345, 459-466, calkpt.F:164)
   const int nx = 2 * T.d1 + 1, ny = 2 * T.d2 + 1;
 #pragma unroll
   for (int v = 0; v < 2; v++) {
-    const int I = i0 + ti + 16 * v;
+    const int I = i0 + il0 + 4 * v;
     if (I >= nv) continue;
     const int k1 = P.kzz[3 * I], k2 = P.kzz[3 * I + 1], k3 = P.kzz[3 * I + 2];
     const double xi = P.xk[I], yi = P.yk[I], zi = P.zk[I];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const int J = j0 + tj + 16 * u;
+      const int J = j0 + jl0 + 8 * u;
       if (J > I) continue;
       const int q = u * 2 + v;
       const double x2 = P.xk[J] * xi + P.yk[J] * yi + P.zk[J] * zi;
@@ -792,10 +879,7 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
 // accumulators of (WT/8)^2 fragments, 4 DMMA per fragment and 4 k), the
 // operand rows of TRI_KC k copied by cp.async three stages deep.  A row of
 // shared memory holds 2 WT + 2 elements: the 8 lanes of a quarter-warp
-// (4 k x 2 i) then read 8 different 16-byte banks.  Measured: 40 atoms (N =
-// 4937, K = 2000) 6.24 ms = 31.5 TFLOP/s against 6.86 for library ZGEMM panels
-// plus an FMA kernel on the diagonal blocks; six atoms (N = 704, K = 300), the
-// update and its LO block 50 us against 138.
+// (4 k x 2 i) then read 8 different 16-byte banks.
 // ---------------------------------------------------------------------
 #define TRI_KC 16
 #define TRI_STAGES 3

@@ -2,7 +2,8 @@
 //
 // Host side: context (stream, events, grow-only device buffers), upload of
 // one k-point's inputs, and the stage sequence of calkpt.F:153-185:
-//   HAMILT  -> k_albl, k_phase, k_table, k_sph_coef, k_spherical, k_lo
+//   HAMILT  -> k_albl, k_phase, k_table, k_sph_coef, k_pair_rows, k_spherical
+//              (or sphtc::k_sph_slice, k_sph_tc), k_lo
 //   ZSWAP   -> folded into the HAMILT writes (diag(HS) = H, HSDIAG = S)
 //   HNS     -> k_hns_alm, k_hns_tmul, k_hns_lo_ops (operands), then
 //              k_tri_gemm (FP64, DMMA) or the split-precision tcgen05 path,
@@ -1117,7 +1118,16 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
       int ntiles = 0;
       const int2* tl = tiles_tri(k, "sph", nv, SPH_T, &ntiles);
       if (!tl) return LAPW1GPU_ERR_NOMEM;
-      if (!c->smem((const void*)k_spherical, SPH_DYN_SMEM)) return LAPW1GPU_ERR_CUDA;
+      const size_t nrow = (size_t)nat * ltop * k->nvpad;
+      double2* rowJ = (double2*)c->sbuf(set, "rowj", sizeof(double2) * nrow);
+      double2* rowI = (double2*)c->sbuf(set, "rowi", 2 * sizeof(double2) * nrow);
+      if (!rowJ || !rowI) return LAPW1GPU_ERR_NOMEM;
+      nl++;
+      k_pair_rows<<<dim3((k->nvpad + 127) / 128, nat * ltop), 128, 0, s>>>(P, coef, rowJ, rowI);
+      const bool lt11 = ltop == PR_LT;
+      const void* fn = lt11 ? (const void*)k_spherical<PR_LT, false> : (const void*)k_spherical<SPH_LMAX, true>;
+      const int smem = sph_smem_bytes(lt11 ? PR_LT : SPH_LMAX);
+      if (!c->smem(fn, smem)) return LAPW1GPU_ERR_CUDA;
       if (ev) CK(cudaEventRecord(ev[12], s));
       // tiles are ordered by the I tile (column of S), bi (bi + 1) / 2 before tile row bi
       const int nbi = (nv + SPH_T - 1) / SPH_T;
@@ -1128,8 +1138,12 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
         const long t0 = (long)b0 * (b0 + 1) / 2, t1 = (long)b1 * (b1 + 1) / 2;
         if (t1 > t0) {
           nl++;
-          k_spherical<<<(unsigned)(t1 - t0), SPH_THREADS, SPH_DYN_SMEM, s>>>(P, tl + t0, coef, tab, k->tab, d_hs,
-                                                                             ldhs, d_hsdiag);
+          if (lt11)
+            k_spherical<PR_LT, false><<<(unsigned)(t1 - t0), SPH_THREADS, smem, s>>>(P, tl + t0, rowJ, rowI, tab, k->tab,
+                                                                                     d_hs, ldhs, d_hsdiag);
+          else
+            k_spherical<SPH_LMAX, true><<<(unsigned)(t1 - t0), SPH_THREADS, smem, s>>>(P, tl + t0, rowJ, rowI, tab,
+                                                                                       k->tab, d_hs, ldhs, d_hsdiag);
         }
         if (sp && sp->col[g + 1] <= nv) {
           CK(cudaEventRecord(sp->sev[g], s));
@@ -1887,14 +1901,14 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
   }
   if (!tl) return LAPW1GPU_ERR_NOMEM;
   const size_t nrow = (size_t)nat * ltop * k->nvpad;
-  double2* rowJ = (double2*)c->buf("frc_rowj", sizeof(double2) * nrow);
-  double2* rowI = (double2*)c->buf("frc_rowi", 2 * sizeof(double2) * nrow);
+  double2* rowJ = (double2*)c->buf("rowj", sizeof(double2) * nrow);
+  double2* rowI = (double2*)c->buf("rowi", 2 * sizeof(double2) * nrow);
   if (!rowJ || !rowI) return LAPW1GPU_ERR_NOMEM;
-  k_force_rows<<<dim3((k->nvpad + 127) / 128, nat * ltop), 128, 0, s>>>(P, coef, rowJ, rowI);
-  nlf += 3;  // k_force_rows, k_force_sph, k_force_step
-  const bool lt11 = ltop == FRC_LT;
-  const void* fsph = lt11 ? (const void*)k_force_sph<FRC_LT, false> : (const void*)k_force_sph<SPH_LMAX, true>;
-  const int fsmem = frc_smem_bytes(lt11 ? FRC_LT : SPH_LMAX);
+  k_pair_rows<<<dim3((k->nvpad + 127) / 128, nat * ltop), 128, 0, s>>>(P, coef, rowJ, rowI);
+  nlf += 3;  // k_pair_rows, k_force_sph, k_force_step
+  const bool lt11 = ltop == PR_LT;
+  const void* fsph = lt11 ? (const void*)k_force_sph<PR_LT, false> : (const void*)k_force_sph<SPH_LMAX, true>;
+  const int fsmem = frc_smem_bytes(lt11 ? PR_LT : SPH_LMAX);
   if (!c->smem(fsph, fsmem)) return LAPW1GPU_ERR_CUDA;
   const size_t nbox = (size_t)(2 * k->tab.d1 + 1) * (2 * k->tab.d2 + 1) * (2 * k->tab.d3 + 1);
   double* bins = (double*)c->buf("frc_bins", sizeof(double) * 2 * nbox);
@@ -1951,7 +1965,7 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
     if (timed) CK(cudaEventRecord(c->fev[6], s));
   }
   if (lt11)
-    k_force_sph<FRC_LT, false><<<ntiles, FRC_THREADS, fsmem, s>>>(P, tl, rowJ, rowI, k->tab, rho, rhoe, n, rt,
+    k_force_sph<PR_LT, false><<<ntiles, FRC_THREADS, fsmem, s>>>(P, tl, rowJ, rowI, k->tab, rho, rhoe, n, rt,
                                                                   d_grad, bins);
   else
     k_force_sph<SPH_LMAX, true><<<ntiles, FRC_THREADS, fsmem, s>>>(P, tl, rowJ, rowI, k->tab, rho, rhoe, n, rt,
