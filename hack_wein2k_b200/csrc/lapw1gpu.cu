@@ -54,6 +54,7 @@ struct DevBuf {
 
 #define L1G_MAX_SETS 4  // concurrent k-point chains in a batch (scratch sets)
 #define L1G_MAX_GROUPS 16
+#define L1G_STAGE_MAX (256u << 10)  // an upload's arrays up to this size go through page-locked staging
 
 // Column groups of HS: the spherical contraction and the HNS update run
 // group by group, each group followed by an event, so that a caller can
@@ -103,6 +104,11 @@ struct lapw1gpu_context {
   bool async_copies = false;                  // HS copies queued on the copy stream (ev[11] ends them)
   int async_nl = 0;
   bool async_pending = false;
+  // page-locked staging of an upload's small arrays and the event that ends
+  // the copy out of it (grow-only, at most the small segments of one problem)
+  void* h_stage = nullptr;
+  size_t h_stage_bytes = 0;
+  cudaEvent_t stage_done = nullptr;
   int prec = LAPW1GPU_PREC_FP64;
   int slices = 5;      // int8 slices of the spherical part (split precision)
   int slices_hns = 5;  // int8 slices of the HNS update
@@ -384,6 +390,7 @@ int lapw1gpu_init(int device, lapw1gpu_context** out) {
     cudaEventCreateWithFlags(&c->auxj[i], cudaEventDisableTiming);
   }
   cudaEventCreateWithFlags(&c->async_done, cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&c->stage_done, cudaEventDisableTiming);
   // status words read back through mapped host memory (a one-thread kernel
   // stores them), not by copies, which would queue behind a running
   // lapw1gpu_setup_async's HS copies on the copy engines
@@ -429,6 +436,8 @@ int lapw1gpu_finalize(lapw1gpu_context* c) {
   if (c->h_async_status) cudaFreeHost(c->h_async_status);
   if (c->h_status) cudaFreeHost(c->h_status);
   if (c->async_done) cudaEventDestroy(c->async_done);
+  if (c->stage_done) cudaEventDestroy(c->stage_done);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
   if (c->d_status) cudaFree(c->d_status);
   for (auto& e : c->ev) cudaEventDestroy(e);
   for (auto& e : c->fev) cudaEventDestroy(e);
@@ -654,19 +663,20 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
         k->orbs.push_back(it);
       }
   }
-  // one arena for all device inputs
+  // One arena for all device inputs (add: the segment's index).  The small
+  // arrays come first in it, gathered in page-locked memory and sent by one
+  // copy: a copy of its own costs each of some 35 arrays about 4 us, more than
+  // a small problem's kernels.  Arrays above L1G_STAGE_MAX are copied from
+  // the caller's memory directly.
   struct Seg {
     const void* src;
     size_t bytes;
     size_t off;
   };
   std::vector<Seg> segs;
-  size_t off = 0;
   auto add = [&](const void* src, size_t bytes) -> size_t {
-    size_t o = off;
-    segs.push_back({src, bytes, o});
-    off += (bytes + 255) / 256 * 256;
-    return o;
+    segs.push_back({src, bytes, 0});
+    return segs.size() - 1;
   };
   const int nat = p->nat, ndf = p->ndf, n = p->n, ldl = p->ldl;
   const int L4 = L1G_LOMAX + 1;
@@ -706,6 +716,15 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   size_t o_locol = add(k->locols.data(), sizeof(LoCol) * std::max<size_t>(1, k->locols.size()));
   size_t o_lor = add(k->loranges.data(), sizeof(LoRange) * std::max<size_t>(1, k->loranges.size()));
   size_t o_pots = add(k->pots.data(), sizeof(double2) * std::max<size_t>(1, k->pots.size()));
+  size_t off = 0, small = 0;  // bytes of the arena, of its small segments
+  for (int pass = 0; pass < 2; pass++) {
+    for (auto& s : segs)
+      if ((s.bytes <= L1G_STAGE_MAX) == (pass == 0)) {
+        s.off = off;
+        off += (s.bytes + 255) / 256 * 256;
+      }
+    if (pass == 0) small = off;
+  }
   if (borrow) {
     // one-shot host entry point: reuse the context's grow-only arena
     k->arena = ctx->buf("arena", off);
@@ -722,11 +741,41 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   k->arena_bytes = off;
   char* base = (char*)k->arena;
   int crc = LAPW1GPU_OK;
+  // the staging buffer, free once the copy out of it (an earlier upload's) is done
+  char* stage = nullptr;
+  if (cudaEventSynchronize(ctx->stage_done) != cudaSuccess) crc = LAPW1GPU_ERR_CUDA;
+  if (crc == LAPW1GPU_OK && ctx->h_stage_bytes < small) {
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    ctx->h_stage = nullptr;
+    ctx->h_stage_bytes = 0;
+    if (cudaHostAlloc(&ctx->h_stage, small, cudaHostAllocDefault) == cudaSuccess) {
+      ctx->h_stage_bytes = small;
+    } else {
+      cudaGetLastError();  // without it every array is copied from the caller's memory
+      ctx->h_stage = nullptr;
+    }
+  }
+  if (ctx->h_stage_bytes >= small) stage = (char*)ctx->h_stage;
+  bool direct = false;  // an array is copied from the caller's memory
   for (auto& s : segs)
-    if (s.src && s.bytes && crc == LAPW1GPU_OK)
-      if (cudaMemcpyAsync(base + s.off, s.src, s.bytes, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-        crc = LAPW1GPU_ERR_CUDA;
-  if (crc == LAPW1GPU_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) crc = LAPW1GPU_ERR_CUDA;
+    if (s.src && s.bytes && crc == LAPW1GPU_OK) {
+      if (stage && s.bytes <= L1G_STAGE_MAX) {
+        memcpy(stage + s.off, s.src, s.bytes);
+      } else {
+        direct = true;
+        if (cudaMemcpyAsync(base + s.off, s.src, s.bytes, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+          crc = LAPW1GPU_ERR_CUDA;
+      }
+    }
+  if (crc == LAPW1GPU_OK && stage && small &&
+      (cudaMemcpyAsync(base, stage, small, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
+       cudaEventRecord(ctx->stage_done, ctx->stream) != cudaSuccess))
+    crc = LAPW1GPU_ERR_CUDA;
+  // an upload that outlives the call must not depend on the caller's arrays
+  // (a copy from page-locked ones may still run); a host setup keeps them
+  // until it ends, and its kernels follow the copies on the stream
+  if (crc == LAPW1GPU_OK && direct && !borrow && cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+    crc = LAPW1GPU_ERR_CUDA;
   if (crc != LAPW1GPU_OK) {
     cudaGetLastError();
     if (k->owns_arena) cudaFree(k->arena);
@@ -746,7 +795,7 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   P.nvpad = k->nvpad;
   P.npad = k->npad;
   P.vi = p->vi;
-#define SEGP(T, o) reinterpret_cast<T>(base + (o))
+#define SEGP(T, o) reinterpret_cast<T>(base + segs[o].off)
   P.mult = SEGP(const int*, o_mult);
   P.atype = SEGP(const int*, o_atype);
   P.afirst = SEGP(const int*, o_afirst);

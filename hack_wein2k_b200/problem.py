@@ -42,6 +42,14 @@ class CProblem(C.Structure):
     ]
 
 
+# array fields of CProblem: name, element type, 8-byte word in the struct
+_ARRAYS = [(name, np.float64 if ctype is _dp else np.int32, getattr(CProblem, name).offset // 8)
+           for name, ctype in CProblem._fields_ if ctype in (_dp, _ip)]
+_ARRAYS = [(name, np.complex128 if name in ("warp", "tns", "vorb") else dtype, word) for name, dtype, word in _ARRAYS]
+# what the orbital fields point to when there are none
+_ORB_EMPTY = dict(iatom=np.zeros(1), nlorb=np.zeros(1), lorb=np.zeros((1, 3)), vorb=np.zeros((1, 4, 7, 7)))
+
+
 class CStats(C.Structure):
     """ctypes mirror of `lapw1gpu_stats`."""
 
@@ -142,8 +150,7 @@ class Problem:
         assert self.rotloc.shape == (nat, 3, 3)
         assert self.p.shape == (nat, self.ldl) and self.ldl >= self.ltop
         assert self.ilo.shape == (nat, LOMAX + 1)
-        nlo = int(sum((2 * l + 1) * self.mult[a] * self.ilo[a, l]
-                      for a in range(nat) for l in range(LOMAX + 1)))
+        nlo = int(np.dot(self.mult, np.dot(self.ilo, 2 * np.arange(LOMAX + 1) + 1)))
         assert nlo == self.nlo, (nlo, self.nlo)
         assert self.tns.shape == (nat, NTNS, NSL2, NSL2)
         assert np.asarray(self.bkzz).shape == (3, 3)
@@ -152,45 +159,24 @@ class Problem:
         """Marshal into the C struct.  The returned struct keeps references
         to the contiguous arrays it points into (attribute `_keep`)."""
         self.validate()
-        keep = []
-
-        def dptr(a):
-            a = np.ascontiguousarray(a, dtype=np.float64)
-            keep.append(a)
-            return a.ctypes.data_as(_dp)
-
-        def cptr(a):
-            a = np.ascontiguousarray(a, dtype=np.complex128)
-            keep.append(a)
-            return a.ctypes.data_as(_dp)
-
-        def iptr(a):
-            a = np.ascontiguousarray(a, dtype=np.int32)
-            keep.append(a)
-            return a.ctypes.data_as(_ip)
-
         w1, w2, w3 = self.warp_half
         s = CProblem(
             n=self.n, nv=self.nv, nlo=self.nlo, nat=self.nat, ndf=self.ndf,
             ltop=self.ltop, ldl=self.ldl, lnsmax=self.lnsmax, ins=self.ins,
             nohns=self.nohns, vi=float(self.vi),
             bkzz=(C.c_double * 9)(*np.asarray(self.bkzz, dtype=np.float64).reshape(9)),
-            mult=iptr(self.mult), rmt=dptr(self.rmt), v=dptr(self.v), pos=dptr(self.pos),
-            rotij=dptr(self.rotij), rotloc=dptr(self.rotloc),
-            kzz=iptr(self.kzz), xk=dptr(self.xk), yk=dptr(self.yk), zk=dptr(self.zk),
-            rk=dptr(self.rk),
-            p=dptr(self.p), pe=dptr(self.pe), dp=dptr(self.dp), dpe=dptr(self.dpe),
-            pei=dptr(self.pei), e=dptr(self.e), lapw=iptr(self.lapw),
-            ilo=iptr(self.ilo), loor=iptr(self.loor), alo=dptr(self.alo), blo=dptr(self.blo),
-            clo=dptr(self.clo), elo=dptr(self.elo), pi12lo=dptr(self.pi12lo),
-            pe12lo=dptr(self.pe12lo), dplo=dptr(self.dplo),
-            warp1=w1, warp2=w2, warp3=w3, warp=cptr(self.warp),
-            tns=cptr(self.tns),
-            natorb=self.natorb, iatom=iptr(self.iatom if self.natorb else np.zeros(1)),
-            nlorb=iptr(self.nlorb if self.natorb else np.zeros(1)),
-            lorb=iptr(self.lorb if self.natorb else np.zeros((1, 3))),
-            vorb=cptr(self.vorb if self.natorb else np.zeros((1, 4, 7, 7))),
-        )
+            warp1=w1, warp2=w2, warp3=w3, natorb=self.natorb)
+        # the array fields' addresses written into the struct as words: a
+        # typed ctypes pointer per array costs several microseconds, some 45
+        # arrays per call
+        words, keep = np.frombuffer(s, dtype=np.uintp), []
+        for name, dtype, word in _ARRAYS:
+            a = getattr(self, name)
+            if name in _ORB_EMPTY and not self.natorb:
+                a = _ORB_EMPTY[name]
+            a = np.ascontiguousarray(a, dtype=dtype)
+            keep.append(a)
+            words[word] = a.__array_interface__["data"][0]
         s._keep = keep
         return s
 
