@@ -1006,132 +1006,80 @@ __global__ void k_add_lower(int nv, int nlo, const double2* __restrict__ T, doub
 }
 
 // ---------------------------------------------------------------------
-// K-orb: HORB (horb.F:98-297) for one (U-atom a, l = lvor)
+// K-orb: HORB (horb.F:98-297).  For U-atom a and l = lvor the reference adds
+//   sum_(alpha,beta) g_(alpha beta) sum_(m0,m1) conj(X_alpha(m0,i)) pot(m1,m0) X_beta(m1,j)
+// to HS(i,j), i >= j, with X = (ALM, BLM, CLM) of the row (CLM only on the
+// atom type's own LO rows of that l, whose ALM, BLM are their LO coefficients;
+// zero on all other LO rows) and g the overlaps of (u, udot, u_lo): g_AA =
+// g_CC = 1, g_BB = PEI, g_AC = PI12LO, g_BC = PE12LO.  (Its cases PW-PW, PW-LO
+// and LO-LO are this sum with the zero parts left out: i >= j puts an LO row j
+// of the same type and l in a block not after i's.)  So all atoms and l
+// together are one product over k = (item, alpha, m0), L[k][i] = conj(X), R[k][j]
+// = the inner sums, which k_tri_gemm adds in one pass over HS.
 // ---------------------------------------------------------------------
-__global__ void k_horb_rows(DevProb P, int a, int lvor, const double2* __restrict__ pot /*[7][7] pot(m2,m1)*/,
-                            const LoRange* __restrict__ lor, int nlor, double2* __restrict__ alm,
-                            double2* __restrict__ blm, double2* __restrict__ clm) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+struct OrbItem {
+  int a, lvor, pot, k0;  // atom, l, its pot(m2,m1) block of 49, first k
+};
+__global__ void k_horb_rows(DevProb P, const OrbItem* __restrict__ items, const double2* __restrict__ pots,
+                            const LoRange* __restrict__ lor, int nlor, double2* __restrict__ L,
+                            double2* __restrict__ R) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.n) return;
+  const OrbItem it = items[blockIdx.y];
+  const int a = it.a, lvor = it.lvor, nm = 2 * lvor + 1;
+  const double2* pot = pots + (size_t)it.pot * 49;  // [7][7] pot(m2,m1)
   const int jn = P.atype[a];
   const double pi = 3.141592653589793238462643;
   const double rhoatm = 4.0 * pi * sqrt(P.vi) * P.rmt[jn] * P.rmt[jn];
   const double* r = P.pos + 3 * a;
-  double arg = (r[0] * P.kzz[3 * i] + r[1] * P.kzz[3 * i + 1] + r[2] * P.kzz[3 * i + 2]);
-  double2 ph = cexp2pi(arg);
+  const double2 ph = cexp2pi(r[0] * P.kzz[3 * i] + r[1] * P.kzz[3 * i + 1] + r[2] * P.kzz[3 * i + 2]);
   double2 y[16];
   dev_ylm_row<3>(P.xk[i], P.yk[i], P.zk[i], P.rotij + 9 * a, P.rotloc + 9 * jn, lvor, y);
   double2 cil = cmk(1.0, 0.0);
   for (int q = 0; q < lvor; q++) cil = cmk(-cil.y, cil.x);
-  int myjlo = 0;
-  if (i >= P.nv) {
-    int li = i - P.nv + 1;
+  // the row's coefficients of (u, udot, u_lo): X = coefficient times t(m)
+  double ca = 0.0, cb = 0.0, cc = 0.0;
+  if (i < P.nv) {
+    const size_t o = ((size_t)jn * P.ltop + lvor) * P.nvpad + i;
+    ca = P.al[o];
+    cb = P.bl[o];
+  } else {
+    const int li = i - P.nv + 1;
+    int myjlo = 0;
     for (int q = 0; q < nlor; q++)
       if (lor[q].jn == jn && lor[q].l == lvor && li >= lor[q].i1 && li <= lor[q].i2) myjlo = lor[q].jlo;
-  }
-  for (int m = -3; m <= 3; m++) {
-    double2 A = cmk(0, 0), B = A, Cc = A;
-    if (m >= -lvor && m <= lvor) {
-      int lm = lvor * (lvor + 1) + m;
-      double2 t1 = cmul(cmul(cscale(cil, rhoatm), ph), cconj(y[lm]));
-      if (i < P.nv) {
-        size_t o = ((size_t)jn * P.ltop + lvor) * P.nvpad + i;
-        A = cscale(t1, P.al[o]);
-        B = cscale(t1, P.bl[o]);
-      } else if (myjlo > 0) {
-        int oo = (jn * L1G_NLOAT + myjlo - 1) * (L1G_LOMAX + 1) + lvor;
-        B = cscale(t1, P.blo[oo]);
-        Cc = cscale(t1, P.clo[oo]);
-        A = cscale(t1, P.alo[oo]);
-      }
+    if (myjlo > 0) {
+      const int oo = (jn * L1G_NLOAT + myjlo - 1) * (L1G_LOMAX + 1) + lvor;
+      ca = P.alo[oo];
+      cb = P.blo[oo];
+      cc = P.clo[oo];
     }
-    alm[(size_t)i * 7 + m + 3] = A;
-    blm[(size_t)i * 7 + m + 3] = B;
-    clm[(size_t)i * 7 + m + 3] = Cc;
   }
-}
-
-__global__ void k_horb_pairs(DevProb P, int a, int lvor, const double2* __restrict__ pot, const LoRange* __restrict__ lor,
-                             int nlor, const double2* __restrict__ alm, const double2* __restrict__ blm,
-                             const double2* __restrict__ clm, double2* __restrict__ hs, int ld) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y;
-  if (i >= P.n || i < j) return;
-  const int jn = P.atype[a], nv = P.nv;
-  const int o = jn * P.ldl + lvor;
-  const double peil = P.pei[o];
+  const double peil = P.pei[jn * P.ldl + lvor];
   const double pi12 = lvor <= L1G_LOMAX ? P.pi12lo[jn * (L1G_LOMAX + 1) + lvor] : 0.0;
   const double pe12 = lvor <= L1G_LOMAX ? P.pe12lo[jn * (L1G_LOMAX + 1) + lvor] : 0.0;
-#define POT(m1, m0) pot[((m1) + 3) * 7 + (m0) + 3]
-#define AL7(mm, r) alm[(size_t)(r)*7 + (mm) + 3]
-#define BL7(mm, r) blm[(size_t)(r)*7 + (mm) + 3]
-#define CL7(mm, r) clm[(size_t)(r)*7 + (mm) + 3]
-  double2 add = cmk(0.0, 0.0);
-  bool hit = false;
-  if (i < nv && j < nv) {
-    double2 t4 = cmk(0, 0), t5 = cmk(0, 0);
-    for (int m0 = -lvor; m0 <= lvor; m0++) {
-      double2 t1 = cmk(0, 0), t2 = cmk(0, 0);
-      for (int m1 = -lvor; m1 <= lvor; m1++) {
-        t1 = cadd(t1, cmul(POT(m1, m0), AL7(m1, j)));
-        t2 = cadd(t2, cmul(POT(m1, m0), BL7(m1, j)));
-      }
-      t2 = cscale(t2, peil);
-      t4 = cadd(t4, cmul(t1, cconj(AL7(m0, i))));
-      t5 = cadd(t5, cmul(t2, cconj(BL7(m0, i))));
-    }
-    add = cadd(t4, t5);
-    hit = true;
-  } else if (i >= nv && lvor <= L1G_LOMAX) {
-    int li = i - nv + 1, lj = j - nv + 1;
-    int jlo_i = 0, i22 = 0, jlo_j = 0;
-    for (int q = 0; q < nlor; q++) {
-      if (lor[q].jn == jn && lor[q].l == lvor && li >= lor[q].i1 && li <= lor[q].i2) jlo_i = lor[q].jlo;
-      if (j >= nv && lor[q].jn == jn && lor[q].l == lvor && lj >= lor[q].i1 && lj <= lor[q].i2) {
-        jlo_j = lor[q].jlo;
-        i22 = lor[q].i2;
-      }
-    }
-    if (jlo_i > 0 && j < nv) {  // <APW||LO>
-      double2 t4 = cmk(0, 0), t5 = t4, t6 = t4, t7 = t4;
-      for (int m0 = -lvor; m0 <= lvor; m0++) {
-        double2 t1 = cmk(0, 0), t2 = cmk(0, 0);
-        for (int m1 = -lvor; m1 <= lvor; m1++) {
-          t1 = cadd(t1, cmul(AL7(m1, j), POT(m1, m0)));
-          t2 = cadd(t2, cmul(BL7(m1, j), POT(m1, m0)));
-        }
-        t4 = cadd(t4, cmul(t1, cconj(AL7(m0, i))));
-        t5 = cadd(t5, cmul(t2, cconj(BL7(m0, i))));
-        t6 = cadd(t6, cmul(t1, cconj(CL7(m0, i))));
-        t7 = cadd(t7, cmul(t2, cconj(CL7(m0, i))));
-      }
-      add = cadd(cadd(cadd(t4, cscale(t5, peil)), cscale(t6, pi12)), cscale(t7, pe12));
-      hit = true;
-    } else if (jlo_i > 0 && jlo_j > 0 && jlo_j <= jlo_i && lj <= i22) {  // <LO||LO>
-      double2 t4 = cmk(0, 0), t5 = t4, t6 = t4, t7 = t4;
-      for (int m0 = -lvor; m0 <= lvor; m0++) {
-        double2 t1 = cmk(0, 0), t2 = t1, t3 = t1;
-        for (int m1 = -lvor; m1 <= lvor; m1++) {
-          t1 = cadd(t1, cmul(POT(m1, m0), AL7(m1, j)));
-          t2 = cadd(t2, cmul(POT(m1, m0), BL7(m1, j)));
-          t3 = cadd(t3, cmul(POT(m1, m0), CL7(m1, j)));
-        }
-        t4 = cadd(cadd(t4, cmul(t1, cconj(AL7(m0, i)))), cmul(cconj(CL7(m0, i)), t3));
-        t5 = cadd(t5, cmul(cconj(BL7(m0, i)), t2));
-        t6 = cadd(cadd(t6, cmul(cconj(CL7(m0, i)), t1)), cmul(cconj(AL7(m0, i)), t3));
-        t7 = cadd(cadd(t7, cmul(cconj(BL7(m0, i)), t3)), cmul(cconj(CL7(m0, i)), t2));
-      }
-      add = cadd(cadd(cadd(cscale(t5, peil), cscale(t6, pi12)), cscale(t7, pe12)), t4);
-      hit = true;
-    }
-  }
-#undef POT
-#undef AL7
-#undef BL7
-#undef CL7
-  if (hit) {
-    double2* dst = hs + (size_t)j * ld + i;
-    *dst = cadd(*dst, add);
+  const double ga = ca + pi12 * cc, gb = peil * cb + pe12 * cc, gc = pi12 * ca + pe12 * cb + cc;
+  const size_t st = P.npad;
+  double2* Li = L + (size_t)it.k0 * st + i;
+  double2* Ri = R + (size_t)it.k0 * st + i;
+  double2 t[7];
+#pragma unroll
+  for (int m = 0; m < 7; m++)
+    if (m < nm) t[m] = cmul(cmul(cscale(cil, rhoatm), ph), cconj(y[lvor * lvor + m]));
+#pragma unroll
+  for (int m0 = 0; m0 < 7; m0++) {
+    if (m0 >= nm) continue;
+    double2 q = cmk(0.0, 0.0);  // sum_m1 pot(m1,m0) t(m1)
+#pragma unroll
+    for (int m1 = 0; m1 < 7; m1++)
+      if (m1 < nm) q = cadd(q, cmul(pot[(m1 + 3 - lvor) * 7 + m0 + 3 - lvor], t[m1]));
+    const double2 tc = cconj(t[m0]);
+    Li[(size_t)m0 * st] = cscale(tc, ca);
+    Li[(size_t)(nm + m0) * st] = cscale(tc, cb);
+    Li[(size_t)(2 * nm + m0) * st] = cscale(tc, cc);
+    Ri[(size_t)m0 * st] = cscale(q, ga);
+    Ri[(size_t)(nm + m0) * st] = cscale(q, gb);
+    Ri[(size_t)(2 * nm + m0) * st] = cscale(q, gc);
   }
 }
 

@@ -210,11 +210,9 @@ struct lapw1gpu_kpoint {
   std::vector<LoCol> locols;
   std::vector<LoRange> loranges;
   std::vector<int> mult, atype, afirst;
-  // HORB description
-  struct OrbItem {
-    int a, lvor, iat;
-  };
+  // HORB description: its items (atom, l) and the products' K
   std::vector<OrbItem> orbs;
+  int korb = 0;
   std::vector<double2> pots;  // [norb][49] pot(m1,m0) arrays
   // device inputs (one arena)
   void* arena = nullptr;
@@ -226,6 +224,7 @@ struct lapw1gpu_kpoint {
   const LoCol* d_locols = nullptr;
   const LoRange* d_loranges = nullptr;
   const double2* d_pots = nullptr;
+  const OrbItem* d_orbs = nullptr;
 };
 
 // Device tile list for the shape named by `key` (sizes and tile parameters),
@@ -659,8 +658,8 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
     }
     for (int e = 0; e < p->mult[jn]; e++)
       for (int q = 0; q < p->nlorb[i]; q++) {
-        lapw1gpu_kpoint::OrbItem it{k->afirst[jn] + e, p->lorb[i * 3 + q], pot0 + q};
-        k->orbs.push_back(it);
+        k->orbs.push_back({k->afirst[jn] + e, p->lorb[i * 3 + q], pot0 + q, k->korb});
+        k->korb += 3 * (2 * p->lorb[i * 3 + q] + 1);
       }
   }
   // One arena for all device inputs (add: the segment's index).  The small
@@ -713,9 +712,10 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   size_t o_warp = add(p->ins == 0 ? (const void*)p->warp : nullptr, p->ins == 0 ? sizeof(double2) * nwarp : 16);
   size_t ntns = (size_t)nat * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2;
   size_t o_tns = add(p->nohns ? nullptr : (const void*)p->tns, p->nohns ? 16 : sizeof(double2) * ntns);
-  size_t o_locol = add(k->locols.data(), sizeof(LoCol) * std::max<size_t>(1, k->locols.size()));
-  size_t o_lor = add(k->loranges.data(), sizeof(LoRange) * std::max<size_t>(1, k->loranges.size()));
-  size_t o_pots = add(k->pots.data(), sizeof(double2) * std::max<size_t>(1, k->pots.size()));
+  size_t o_locol = add(k->locols.data(), sizeof(LoCol) * k->locols.size());
+  size_t o_lor = add(k->loranges.data(), sizeof(LoRange) * k->loranges.size());
+  size_t o_pots = add(k->pots.data(), sizeof(double2) * k->pots.size());
+  size_t o_orbs = add(k->orbs.data(), sizeof(OrbItem) * k->orbs.size());
   size_t off = 0, small = 0;  // bytes of the arena, of its small segments
   for (int pass = 0; pass < 2; pass++) {
     for (auto& s : segs)
@@ -830,6 +830,7 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   k->d_locols = SEGP(const LoCol*, o_locol);
   k->d_loranges = SEGP(const LoRange*, o_lor);
   k->d_pots = SEGP(const double2*, o_pots);
+  k->d_orbs = SEGP(const OrbItem*, o_orbs);
 #undef SEGP
   *out = k;
   return LAPW1GPU_OK;
@@ -1271,27 +1272,22 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
   if (ev) CK(cudaEventRecord(ev[4], s));
 
   if ((stages & 4) && !k->orbs.empty()) {
-    double2* alm = (double2*)c->sbuf(set, "orb_alm", sizeof(double2) * 7 * (size_t)n);
-    double2* blm = (double2*)c->sbuf(set, "orb_blm", sizeof(double2) * 7 * (size_t)n);
-    double2* clm = (double2*)c->sbuf(set, "orb_clm", sizeof(double2) * 7 * (size_t)n);
-    if (!alm || !blm || !clm) return LAPW1GPU_ERR_NOMEM;
-    for (auto& it : k->orbs) {
-      const double2* pot = k->d_pots + (size_t)it.iat * 49;
-      nl++;
-      k_horb_rows<<<(n + 127) / 128, 128, 0, s>>>(P, it.a, it.lvor, pot, k->d_loranges, (int)k->loranges.size(), alm,
-                                                  blm, clm);
-      nl++;
-      k_horb_pairs<<<dim3((n + 127) / 128, n), 128, 0, s>>>(P, it.a, it.lvor, pot, k->d_loranges,
-                                                           (int)k->loranges.size(), alm, blm, clm, d_hs, ldhs);
-    }
+    const size_t bytes = sizeof(double2) * (size_t)k->korb * k->npad;
+    double2* oL = (double2*)c->sbuf(set, "orbL", bytes);
+    double2* oR = (double2*)c->sbuf(set, "orbR", bytes);
+    if (!oL || !oR) return LAPW1GPU_ERR_NOMEM;
+    nl++;
+    k_horb_rows<<<dim3((n + 127) / 128, (unsigned)k->orbs.size()), 128, 0, s>>>(
+        P, k->d_orbs, k->d_pots, k->d_loranges, (int)k->loranges.size(), oL, oR);
+    if (int rc = launch_tri(c, n, 0, n, k->korb, oL, k->npad, oR, k->npad, d_hs, ldhs, 0, c->d_status, s, &nl)) return rc;
     CK(cudaGetLastError());
   }
   if (ev) CK(cudaEventRecord(ev[5], s));
   // Non-finite elements: the split path's writers (k_sph_tc, k_lo, the
-  // split HNS epilogue, k_add_lower) check what they write; the scan of HS
-  // and HSDIAG is needed when the spherical stage did not run (HS came from
-  // the caller), ran on the FP64 kernel, or HORB added to it.
-  const bool checked = sph_tc_used && !((stages & 4) && !k->orbs.empty());
+  // split HNS epilogue, k_add_lower) and HORB's product check what they
+  // write; the scan of HS and HSDIAG is needed when the spherical stage did
+  // not run (HS came from the caller) or ran on the FP64 kernel.
+  const bool checked = sph_tc_used;
   if (!checked) {
     nl++;
     k_check_finite<<<1184, 256, 0, s>>>(n, d_hs, ldhs, d_hsdiag, c->d_status);
