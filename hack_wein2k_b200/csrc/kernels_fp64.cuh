@@ -807,19 +807,21 @@ __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int n
 // One thread per (la, 4 LO rows) of an atom: block (32 la, 8) over 32 rows,
 // the rows' ALM, BLM, CLM staged in shared memory; each T element read is
 // used for the 4 rows.
-// cj: Lop holds conj(L) (the library product of the split path), so the
-// LO terms are added conjugated.
+// An LO row has ALM, BLM, CLM on the atoms of its own type only: a block
+// whose rows are all zero on the atom writes C2 = 0 and leaves L as it is (39
+// of 40 blocks at 40 types); the T elements of 5 b are loaded together (one b
+// at a time each waited for its own, 27 us for 72 rows).
 #define LOOPS_ROWS 32
 __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __restrict__ tns,
                                                     double2* __restrict__ Lop, const double2* __restrict__ Rop,
-                                                    const double2* __restrict__ Clo, double2* __restrict__ C2lo,
-                                                    int cj) {
+                                                    const double2* __restrict__ Clo, double2* __restrict__ C2lo) {
   __shared__ double2 sX[LOOPS_ROWS][3][L1G_NSL2];
   const int la = threadIdx.x, cy = threadIdx.y;
   const int c0 = blockIdx.x * LOOPS_ROWS;  // first LO row of the block
   const int a = blockIdx.y;
   const int nsl2 = (P.lnsmax + 1) * (P.lnsmax + 1);
   const size_t npad = P.npad;
+  bool some = false;  // a non-zero (or NaN) coefficient of the block's rows on this atom
   for (int q = threadIdx.y * 32 + threadIdx.x; q < LOOPS_ROWS * 3 * nsl2; q += 256) {
     const int r = q / (3 * nsl2), w = (q / nsl2) % 3, b = q % nsl2;
     const int cc = c0 + r;
@@ -832,13 +834,20 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
         v = Clo[((size_t)a * nsl2 + b) * P.nlo + cc];
     }
     sX[r][w][b] = v;
+    some |= v.x != 0.0 || v.y != 0.0;
   }
-  __syncthreads();
+  if (!__syncthreads_or(some)) {
+    if (la < nsl2)
+      for (int c = c0 + cy; c < min(P.nlo, c0 + LOOPS_ROWS); c += 8)
+        C2lo[((size_t)a * nsl2 + la) * P.nlo + c] = cmk(0.0, 0.0);
+    return;
+  }
   if (la >= nsl2 || c0 + cy >= P.nlo) return;
   const double2* T = tns + (size_t)P.atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2;
   double2 da[4], db[4], dc[4];
 #pragma unroll
   for (int u = 0; u < 4; u++) da[u] = db[u] = dc[u] = cmk(0, 0);
+#pragma unroll 5
   for (int b = 0; b < nsl2; b++) {
 #define TT(blk) __ldg(T + ((size_t)(blk)*L1G_NSL2 + la) * L1G_NSL2 + b)
     const double2 tuu21 = TT(2), tud21 = TT(5), tuu12 = TT(6), tdu12 = TT(7), tuu22 = TT(8);
@@ -859,8 +868,8 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
     const size_t i = P.nv + c;
     double2* LA = Lop + ((size_t)(a * 2 + 0) * nsl2 + la) * npad + i;
     double2* LB = Lop + ((size_t)(a * 2 + 1) * nsl2 + la) * npad + i;
-    *LA = cadd(*LA, cj ? cconj(da[u]) : da[u]);
-    *LB = cadd(*LB, cj ? cconj(db[u]) : db[u]);
+    *LA = cadd(*LA, da[u]);
+    *LB = cadd(*LB, db[u]);
     C2lo[((size_t)a * nsl2 + la) * P.nlo + c] = dc[u];
   }
 }

@@ -897,7 +897,7 @@ static int launch_hns_ops(lapw1gpu_context* c, const DevProb& P, const double2* 
   *nl += 2;
   if (P.nlo > 0) {
     k_hns_lo_ops<<<dim3((P.nlo + LOOPS_ROWS - 1) / LOOPS_ROWS, P.ndf), dim3(32, 8), 0, s>>>(P, tns, Lop, Rop, Clo,
-                                                                                           C2lo, 0);
+                                                                                           C2lo);
     *nl += 1;
   }
   return l1g_launch_status(__FILE__, __LINE__);
@@ -2016,7 +2016,8 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
     k_force_sph<SPH_LMAX, true><<<ntiles, FRC_THREADS, fsmem, s>>>(P, tl, rowJ, rowI, k->tab, rho, rhoe, n, rt,
                                                                    d_grad, bins);
   if (timed) CK(cudaEventRecord(c->fev[3], s));
-  k_force_step<<<ndf, 256, 0, s>>>(P, k->tab, bins, d_grad);
+  k_force_step<<<dim3(ndf, std::max(1, std::min((int)((nbox + 255) / 256), 8 * c->nsm / ndf))), 256, 0, s>>>(P, k->tab,
+                                                                                                          bins, d_grad);
   CK(cudaGetLastError());
   if (nlo > 0) {
     k_force_lo<<<dim3((n + 127) / 128, nlo), 128, 0, s>>>(P, k->d_locols, rho, rhoe, n, rt, d_grad);

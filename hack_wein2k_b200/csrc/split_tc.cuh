@@ -179,17 +179,21 @@ struct Cfg {
 // Row exponents for the slicing, in parallel over rows and K chunks:
 // ex[row] = max over k of ilogb(max(|Re|, |Im|)) + 1 (ex starts at a very
 // negative value, so all-zero rows keep a zero scale).  One thread per row,
-// 64 k per block.
+// ROWEXP_K k per block, loaded together.  Bound by the read of X; with 64 k per
+// block in turn a small operand (900 k, 1664 rows) took 18 us of load latency.
+#define ROWEXP_K 16
 __global__ void __launch_bounds__(128) k_rowexp(const double2* __restrict__ X, int Kc, int npad,
                                                 int* __restrict__ ex) {
   const int row = blockIdx.x * 128 + threadIdx.x;
-  const int k0 = blockIdx.y * 64;
+  const int k0 = blockIdx.y * ROWEXP_K;
   if (row >= npad) return;
+  double2 v[ROWEXP_K];
+#pragma unroll
+  for (int q = 0; q < ROWEXP_K; q++)
+    v[q] = k0 + q < Kc ? X[(size_t)(k0 + q) * npad + row] : make_double2(0.0, 0.0);
   double m = 0.0;
-  for (int k = k0; k < min(Kc, k0 + 64); k++) {
-    const double2 v = X[(size_t)k * npad + row];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-  }
+#pragma unroll
+  for (int q = 0; q < ROWEXP_K; q++) m = fmax(m, fmax(fabs(v[q].x), fabs(v[q].y)));
   if (m > 0.0) atomicMax(&ex[row], ilogb(m) + 1);
 }
 
@@ -513,7 +517,7 @@ static int split_gemm_launch(lapw1gpu_context* c, lapw1gpu_kpoint* k, int set, i
     if (cudaMemsetAsync(exA, 0x80, sizeof(int) * np, s) != cudaSuccess ||
         cudaMemsetAsync(exB, 0x80, sizeof(int) * np, s) != cudaSuccess)
       return LAPW1GPU_ERR_CUDA;
-    const dim3 ge((npad + 127) / 128, (Kc + 63) / 64), gs(np / 32, Kcp / 64);
+    const dim3 ge((npad + 127) / 128, (Kc + ROWEXP_K - 1) / ROWEXP_K), gs(np / 32, Kcp / 64);
     split::k_rowexp<<<ge, 128, 0, s>>>(Lop, Kc, npad, exA);
     split::k_rowexp<<<ge, 128, 0, s>>>(Rop, Kc, npad, exB);
     split::k_slice_rows<S><<<gs, 256, 0, s>>>(Lop, Kc, Kcp, npad, np, 0, cjL, exA, A, c->d_status);
@@ -587,8 +591,8 @@ static int split_gemm_rect(lapw1gpu_context* c, lapw1gpu_kpoint* k, int set, int
   if (cudaMemsetAsync(exA, 0x80, sizeof(int) * npL, s) != cudaSuccess ||
       cudaMemsetAsync(exB, 0x80, sizeof(int) * npR, s) != cudaSuccess)
     return LAPW1GPU_ERR_CUDA;
-  split::k_rowexp<<<dim3((npadL + 127) / 128, (Kc + 63) / 64), 128, 0, s>>>(Lop, Kc, npadL, exA);
-  split::k_rowexp<<<dim3((npadR + 127) / 128, (Kc + 63) / 64), 128, 0, s>>>(Rop, Kc, npadR, exB);
+  split::k_rowexp<<<dim3((npadL + 127) / 128, (Kc + ROWEXP_K - 1) / ROWEXP_K), 128, 0, s>>>(Lop, Kc, npadL, exA);
+  split::k_rowexp<<<dim3((npadR + 127) / 128, (Kc + ROWEXP_K - 1) / ROWEXP_K), 128, 0, s>>>(Rop, Kc, npadR, exB);
   split::k_slice_rows<S><<<dim3(npL / 32, Kcp / 64), 256, 0, s>>>(Lop, Kc, Kcp, npadL, npL, 0, 0, exA, A, c->d_status);
   split::k_slice_rows<S><<<dim3(npR / 32, Kcp / 64), 256, 0, s>>>(Rop, Kc, Kcp, npadR, npR, 1, 0, exB, B, c->d_status);
   *nlaunch += 4;
