@@ -20,7 +20,7 @@
 //                 step-function term 3 V BESR of each atom (k_table) depends
 //                 on the pair only through dK, so the pairs are binned by dK
 //                 and k_force_step sums the bins per atom
-//   k_force_rsph, k_force_pre, k_force_bins  (split precision) the PW x PW
+//   fsp_tc.cuh, k_force_bins  (split precision) the PW x PW
 //                 pairs of two different row blocks as int8 projections by
 //                 the addition theorem, against a running prefix; the pairs
 //                 inside a block stay on k_force_sph (see below k_force_step)
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(256) k_force_step(DevProb P, TabDesc T, const 
 // are the projections of block p (Y) against the sum of the projections of
 // the blocks before it (the prefix P), the pairs inside a block go through
 // k_force_sph on the diagonal tiles.  The projections are int8 slice
-// products (k_split_gemm) of the left operand of k_force_rsph with (G c)^T.
+// products, formed and contracted in fsp_tc.cuh.
 // Rows whose |k| is 0 use the direction z (their al, bl vanish for l > 0).
 // The pair kernel uses P_l = x P_(l-1) for |x| >= 0.9999999 (hamilt.F's
 // UTOP branch); the projections use P_l itself (the same value at |x| = 1).
@@ -424,45 +424,6 @@ __device__ __forceinline__ int frc_lof(int lm) {
   return l;
 }
 
-// Left operand of the projections, k-major: row I < NV of Lt (stride ld)
-// holds, at r = (a 2 + alpha) ltop^2 + lm, A^alpha_(t l)(I) Z_lm(k_I)
-// conj(phase_a(I)) for atom a of type t (alpha 0: al, 1: bl).  One block
-// per row.
-__global__ void __launch_bounds__(256) k_force_rsph(DevProb P, double2* __restrict__ Lt, int ld) {
-  __shared__ double z[L1G_MAXL * L1G_MAXL];
-  __shared__ unsigned char lof[L1G_MAXL * L1G_MAXL];
-  const int I = blockIdx.x;
-  const int L2 = P.ltop * P.ltop;
-  if ((int)threadIdx.x < L2) {
-    double ux = 0.0, uy = 0.0, uz = 1.0;
-    const double r = P.rk[I];
-    if (r > 0.0) {
-      ux = P.xk[I] / r;
-      uy = P.yk[I] / r;
-      uz = P.zk[I] / r;
-    }
-    const int lm = threadIdx.x, l = frc_lof(lm);
-    z[lm] = frc_zlm(ux, uy, uz, l, lm - l * l - l);
-    lof[lm] = (unsigned char)l;
-  }
-  __syncthreads();
-  const int per = 2 * L2, K = P.ndf * per;
-  double2* out = Lt + (size_t)I * ld;
-  for (int r = threadIdx.x; r < K; r += blockDim.x) {
-    const int a = r / per, rem = r - a * per, alpha = rem >= L2 ? 1 : 0, lm = rem - alpha * L2;
-    const size_t o = ((size_t)P.atype[a] * P.ltop + lof[lm]) * P.nvpad + I;
-    const double v = (alpha ? P.bl[o] : P.al[o]) * z[lm];
-    const double2 ph = P.phase[(size_t)a * P.npad + I];
-    out[r] = cmk(v * ph.x, -v * ph.y);
-  }
-}
-
-// One block of rows against the prefix: Y and Pre are K x 4nb column-major
-// (stride ld; column g nb + b: g = 0 the plain projection of band b, g =
-// 1..3 the kappa_g-weighted one), rows r = (a 2 + alpha) ltop^2 + lm.
-// Adds block p's cross-block pair sums to F and, with update, Pre += Y.
-// One block per (atom, FRC_PB bands); thread = lm, both alpha rows.
-#define FRC_PB 8
 // the default (lapw1gpu_set_force_projection slices -1): 6 slices (at 5 the
 // c1 adjoint's error grew from 2.5e-8 to 1.2e-5 of its largest component),
 // on when the PW rows span 6 blocks (at c1, 4.5 blocks of 1024 rows, the
@@ -470,70 +431,6 @@ __global__ void __launch_bounds__(256) k_force_rsph(DevProb P, double2* __restri
 // 11.6 blocks, 57.3 against 73.7 ms for the whole adjoint)
 #define L1G_FSP_SLICES 6
 #define L1G_FSP_MIN_BLOCKS 6
-__global__ void __launch_bounds__(128) k_force_pre(DevProb P, const SphCoef* __restrict__ coef,
-                                                   const double2* __restrict__ Y, double2* __restrict__ Pre, int ld,
-                                                   int nb, const double* __restrict__ f,
-                                                   const double* __restrict__ eps, int update,
-                                                   double* __restrict__ F) {
-  __shared__ double red[4][3];
-  const int a = blockIdx.x, b0 = blockIdx.y * FRC_PB, b1 = min(nb, b0 + FRC_PB);
-  const int L2 = P.ltop * P.ltop, t = P.atype[a];
-  double acc[3] = {0.0, 0.0, 0.0};
-  for (int lm = threadIdx.x; lm < L2; lm += blockDim.x) {
-    const SphCoef cf = coef[t * P.ltop + frc_lof(lm)];
-    const double hAA = cf.vif * cf.mAA, hAB = cf.vif * cf.mAB, hBA = cf.vif * cf.mBA, hBB = cf.vif * cf.mBB;
-    const double sAA = cf.vif, sBB = cf.vif * cf.chn;
-    const size_t r0 = (size_t)a * 2 * L2 + lm, r1 = r0 + L2;
-    for (int b = b0; b < b1; b++) {
-      double2 p[2][4], y[2][4];
-#pragma unroll
-      for (int g = 0; g < 4; g++) {
-        const size_t o = (size_t)(g * nb + b) * ld;
-        p[0][g] = Pre[o + r0];
-        p[1][g] = Pre[o + r1];
-        y[0][g] = Y[o + r0];
-        y[1][g] = Y[o + r1];
-      }
-      const double fb = f[b], fe = f[b] * eps[b];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        double X[2][2];
-#pragma unroll
-        for (int al = 0; al < 2; al++)
-#pragma unroll
-          for (int be = 0; be < 2; be++) {
-            // Im(p conj(y)) = p.y y.x - p.x y.y
-            const double2 p0 = p[al][0], pk = p[al][c + 1], y0 = y[be][0], yk = y[be][c + 1];
-            X[al][be] = fma(p0.y, yk.x, -(p0.x * yk.y)) - fma(pk.y, y0.x, -(pk.x * y0.y));
-          }
-        const double tH = fma(hAA, X[0][0], fma(hAB, X[0][1], fma(hBA, X[1][0], hBB * X[1][1])));
-        const double tS = fma(sAA, X[0][0], sBB * X[1][1]);
-        acc[c] = fma(-2.0, fma(fb, tH, -(fe * tS)), acc[c]);
-      }
-      if (update) {
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-          const size_t o = (size_t)(g * nb + b) * ld;
-          Pre[o + r0] = cadd(p[0][g], y[0][g]);
-          Pre[o + r1] = cadd(p[1][g], y[1][g]);
-        }
-      }
-    }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    double v = acc[c];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][c] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    double v = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += red[w][threadIdx.x];
-    atomicAdd(&F[a * 3 + threadIdx.x], v);
-  }
-}
 
 // The step-function bins of k_force_sph alone, for the tiles whose pairs
 // the projections cover (same thread-to-pair map, same bins).

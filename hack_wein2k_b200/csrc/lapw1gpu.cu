@@ -84,7 +84,7 @@ struct lapw1gpu_context {
   float fms[7] = {};        // its intervals (ms), read by lapw1gpu_forces_stats; [5] the projections,
                             // [6] their products (the split_rect_gemm calls)
   bool fproj_last = false;  // the last forces call formed spherical projections
-  std::vector<cudaEvent_t> fpev;  // timed forces call: around each projection product
+  std::vector<cudaEvent_t> fpev;  // timed forces call: around each chunk of the projections
   int fpev_used = 0;
   // per scratch set: the stream that prepares the split HNS operands while
   // the spherical stage runs, and its fork/join events
@@ -265,6 +265,7 @@ static const int2* kp_tiles(lapw1gpu_kpoint* k, const std::string& key, int* cou
 
 #include "split_tc.cuh"
 #include "sph_tc.cuh"
+#include "fsp_tc.cuh"
 
 namespace {
 
@@ -1845,6 +1846,87 @@ int lapw1gpu_setup(lapw1gpu_context* c, const lapw1gpu_problem* p, double* hs, i
   return lapw1gpu_setup_stages(c, p, 7, hs, ldhs, hsdiag, st);
 }
 
+// The spherical projections of all atoms (fsp_tc.cuh) on stream s.  The int8
+// operands of as many atoms as L1G_FSP_BYTES holds are built at a time (half
+// of it again and again where that much cannot be allocated).  timed: events
+// around each chunk's operands and products.
+#ifndef L1G_FSP_BYTES
+#define L1G_FSP_BYTES (16ull << 30)
+#endif
+extern "C++" {
+template <int S>
+static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& P, const SphCoef* coef,
+                        const double* zt, const double2* C, int ldc, int nb, const int* exC, int fB,
+                        const double* d_occ, const double* d_eps, double* d_grad, cudaStream_t s, int* nl, bool timed) {
+  using Cf = fsptc::Cfg<S>;
+  const int nv = k->nv, ndf = k->ndf, MT = (k->ltop * k->ltop + fsptc::LMT - 1) / fsptc::LMT;
+  const int nblk = (nv + fB - 1) / fB, fBp = round_up(fB, 64), Kp = nblk * fBp;
+  const int BT = (nb + Cf::NB - 1) / Cf::NB, nbp = BT * Cf::NB;
+  const size_t typeA = (size_t)S * MT * 128 * Kp, atomB = (size_t)S * 2 * nbp * Kp;
+  // atoms [at[i], at[i+1]) per chunk; left operands of the types they span
+  std::vector<int> at;
+  int8_t *A = nullptr, *B = nullptr;
+  int* exA = nullptr;
+  for (size_t budget = L1G_FSP_BYTES;; budget /= 2) {
+    size_t needA = 0, needB = 0;
+    at.assign(1, 0);
+    for (int a0 = 0; a0 < ndf;) {
+      int a1 = a0 + 1;
+      auto bytes = [&](int e) { return (size_t)(k->atype[e - 1] - k->atype[a0] + 1) * typeA + (size_t)(e - a0) * atomB; };
+      while (a1 < ndf && bytes(a1 + 1) <= budget) a1++;
+      needA = std::max(needA, (size_t)(k->atype[a1 - 1] - k->atype[a0] + 1));
+      needB = std::max(needB, (size_t)(a1 - a0));
+      at.push_back(a0 = a1);
+    }
+    A = (int8_t*)c->buf("fspA", needA * typeA);
+    B = A ? (int8_t*)c->buf("fspB", needB * atomB) : nullptr;
+    exA = B ? (int*)c->buf("fspExA", sizeof(int) * needA * MT * 128 * nblk) : nullptr;
+    if (exA) break;
+    if ((int)at.size() == ndf + 1) return LAPW1GPU_ERR_NOMEM;  // one atom at a time already
+  }
+  if (!c->smem((const void*)fsptc::k_fsp_gemm<S>, Cf::SMEM)) return LAPW1GPU_ERR_CUDA;
+  for (size_t q = 0; q + 1 < at.size(); q++) {
+    const int a0 = at[q], na = at[q + 1] - a0, t0 = k->atype[a0], nt = k->atype[a0 + na - 1] - t0 + 1;
+    const size_t rowsA = (size_t)nt * MT * 128, rowsB = (size_t)na * 2 * nbp;
+    if (timed) {
+      while (c->fpev.size() < 2 * (q + 1)) {
+        cudaEvent_t e;
+        CK(cudaEventCreate(&e));
+        c->fpev.push_back(e);
+      }
+      CK(cudaEventRecord(c->fpev[2 * q], s));
+    }
+    fsptc::k_fsp_left<S><<<dim3(nblk, MT * fsptc::LMT, nt), 256, 0, s>>>(P, zt, t0, fB, fBp, Kp, rowsA, A, exA,
+                                                                       c->d_status);
+    fsptc::k_fsp_right<S><<<dim3(nblk, nbp / 8, na), 256, 0, s>>>(P, C, ldc, nb, nbp, a0, fB, fBp, Kp, rowsB, exC, B,
+                                                               c->d_status);
+    CUtensorMap ta, tb;
+    if (l1g_tmap_3d(&ta, A, Kp, rowsA, S, 128) || l1g_tmap_3d(&tb, B, Kp, rowsB, S, Cf::N)) return LAPW1GPU_ERR_CUDA;
+    fsptc::k_fsp_gemm<S><<<dim3(BT, MT, na), Cf::THREADS, Cf::SMEM, s>>>(
+        ta, tb, P, coef, a0, t0, nblk, fB, fBp, nb, nbp, exA, exC, d_occ, d_eps, d_grad, c->d_status);
+    *nl += 3;
+    if (int rc = l1g_launch_status(__FILE__, __LINE__)) return rc;
+    if (timed) {
+      CK(cudaEventRecord(c->fpev[2 * q + 1], s));
+      c->fpev_used = 2 * (int)(q + 1);
+    }
+  }
+  return LAPW1GPU_OK;
+}
+static int fsp_dispatch(int slices, lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& P, const SphCoef* coef,
+                        const double* zt, const double2* C, int ldc, int nb, const int* exC, int fB,
+                        const double* d_occ, const double* d_eps, double* d_grad, cudaStream_t s, int* nl, bool timed) {
+  switch (slices) {
+    case 4: return fsp_products<4>(c, k, P, coef, zt, C, ldc, nb, exC, fB, d_occ, d_eps, d_grad, s, nl, timed);
+    case 5: return fsp_products<5>(c, k, P, coef, zt, C, ldc, nb, exC, fB, d_occ, d_eps, d_grad, s, nl, timed);
+    case 6: return fsp_products<6>(c, k, P, coef, zt, C, ldc, nb, exC, fB, d_occ, d_eps, d_grad, s, nl, timed);
+    case 7: return fsp_products<7>(c, k, P, coef, zt, C, ldc, nb, exC, fB, d_occ, d_eps, d_grad, s, nl, timed);
+    case 8: return fsp_products<8>(c, k, P, coef, zt, C, ldc, nb, exC, fB, d_occ, d_eps, d_grad, s, nl, timed);
+    default: return LAPW1GPU_ERR_RANGE;
+  }
+}
+}  // extern "C++"
+
 // The adjoint of one k-point queued on the context's stream (no host
 // synchronisation): status bits go to c->d_status, which the caller clears.
 // timed: record the interval events of lapw1gpu_forces_stats.
@@ -1905,7 +1987,7 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
   }
   if (timed) CK(cudaEventRecord(c->fev[1], s));
   // G c (k_force_gscale) and, in split precision, its k-major copy (G c)^T:
-  // the right operand of the spherical and of the HNS projections
+  // the right operand of the HNS projections
   double2* GC = nullptr;
   double2* Gt = nullptr;
   auto make_gc = [&](bool with_gt) -> int {
@@ -1961,40 +2043,14 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
   CK(cudaMemsetAsync(bins, 0, sizeof(double) * 2 * nbox, s));
   if (timed) CK(cudaEventRecord(c->fev[2], s));
   if (fproj) {
-    const int L2 = ltop * ltop, Ks = ndf * 2 * L2, nblk = (nv + fB - 1) / fB;
-    double2* Ls = (double2*)c->buf("frc_ls", sizeof(double2) * (size_t)nv * Ks);
-    double2* Pre = (double2*)c->buf("frc_pre", sizeof(double2) * (size_t)Ks * 4 * nb);
-    double2* Yp = (double2*)c->buf("frc_yp", sizeof(double2) * (size_t)Ks * 4 * nb);
-    if (!Ls || !Pre || !Yp) return LAPW1GPU_ERR_NOMEM;
-    if (int rc = make_gc(true)) return rc;
-    k_force_rsph<<<nv, 256, 0, s>>>(P, Ls, Ks);
-    nlf++;
-    for (int pb = 0; pb < nblk; pb++) {
-      const int r0 = pb * fB, kc = std::min(fB, nv - r0);
-      int nly = 0;
-      if (timed) {
-        while ((int)c->fpev.size() < 2 * (pb + 1)) {
-          cudaEvent_t e;
-          CK(cudaEventCreate(&e));
-          c->fpev.push_back(e);
-        }
-        CK(cudaEventRecord(c->fpev[2 * pb], s));
-      }
-      // block 0 is the first prefix; later blocks are contracted with it
-      int rc = split_rect_gemm(c, k, 0, Ks, 4 * nb, kc, Ls + (size_t)r0 * Ks, Ks, Gt + (size_t)r0 * 4 * nb, 4 * nb,
-                               pb == 0 ? Pre : Yp, Ks, fS, s, &nly, 1, "fsp");
-      if (rc) return rc;
-      if (timed) {
-        CK(cudaEventRecord(c->fpev[2 * pb + 1], s));
-        c->fpev_used = 2 * (pb + 1);
-      }
-      nlf += nly;
-      if (pb > 0) {
-        k_force_pre<<<dim3(ndf, (nb + FRC_PB - 1) / FRC_PB), 128, 0, s>>>(P, coef, Yp, Pre, Ks, nb, d_occ, d_eps,
-                                                                          pb + 1 < nblk ? 1 : 0, d_grad);
-        nlf++;
-      }
-    }
+    const int L2 = ltop * ltop, nblk = (nv + fB - 1) / fB;
+    double* zt = (double*)c->buf("fsp_z", sizeof(double) * (size_t)L2 * k->nvpad);
+    int* exC = (int*)c->buf("fsp_exc", sizeof(int) * (size_t)nb * nblk);
+    if (!zt || !exC) return LAPW1GPU_ERR_NOMEM;
+    fsptc::k_fsp_zlm<<<dim3((nv + 127) / 128, L2), 128, 0, s>>>(P, zt);
+    fsptc::k_fsp_cexp<<<dim3(nblk, nb), 256, 0, s>>>(nv, nb, fB, C, ldc, exC);
+    nlf += 2;
+    if (int rc = fsp_dispatch(fS, c, k, P, coef, zt, C, ldc, nb, exC, fB, d_occ, d_eps, d_grad, s, &nlf, timed)) return rc;
     int nto = 0;
     const int2* to = kp_tiles(k, "fsp_out:" + std::to_string(nv) + ":" + std::to_string(fB), &nto,
                               [&](std::vector<int2>& t) {
