@@ -726,16 +726,28 @@ __device__ __forceinline__ void l1g_cp_wait_all() {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// c += a b for one 8 x 8 tile and 4 k: lane holds a(lane / 4, lane % 4),
+// b(lane % 4, lane / 4), c(lane / 4, 2 (lane % 4) + {0, 1})
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
 #define TMUL_I 64        // columns (basis rows i) per work item
-#define TMUL_ROWS 10     // rows of L per thread (one warp: 10 rows x 64 columns)
-#define TMUL_WARPS 5     // 5 x 10 >= 2 NSL2 = 50 rows
-#define TMUL_SMEM ((2 * L1G_NSL2) * (2 * L1G_NSL2) * 16 + (2 * L1G_NSL2) * TMUL_I * 16)
+#define TMUL_WARPS 4     // 16 columns each
+#define TMUL_MF 7        // 8-row fragments: 56 >= 2 NSL2 = 50 rows
+#define TMUL_KP 52       // k padded to whole steps of 4
+#define TMUL_MS 52       // row strides in shared memory: the 8 lanes of a quarter-warp
+#define TMUL_RS 66       // (4 k x 2 rows or columns) read 8 different 16-byte banks
+#define TMUL_SMEM ((8 * TMUL_MF * TMUL_MS + TMUL_KP * TMUL_RS) * 16)
 // L[(a, r_out, la)][i] = sum_{(r, b)} M[(r_out, la)][(r, b)] conj(R[(a, r, b)][i])
-// A work item is (atom, 64 columns i); block b takes the contiguous items
-// [b per, (b+1) per) (one atom for most of them: M is staged again only
-// when the atom changes).  Thread (warp w, lane): rows 10 w .. 10 w + 9 and
-// columns lane, lane + 32 of the item, 20 complex accumulators; per k two
-// R values (conflict-free rows of smem) and ten broadcast M values.
+// on the FP64 tensor cores.  A work item is (atom, 64 columns i); block b
+// takes the contiguous items [b per, (b+1) per) (one atom for most of them: M
+// is staged again only when the atom changes).  A warp forms all rows of 16
+// columns, 7 x 2 complex fragments; two blocks per SM, so that one stages while
+// the other multiplies.  Measured: 40 atoms (N = 4937) 0.20 ms, 100 atoms (N =
+// 12677) 1.19 ms, 25 GFLOP (20 accumulators per thread on the FMA pipe: 0.29 and
+// 1.80).
 __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int nsl2, int ndf, int per,
                                                               const int* __restrict__ atype,
                                                               const double2* __restrict__ tns,
@@ -743,61 +755,71 @@ __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int n
                                                               double2* __restrict__ Lop) {
   extern __shared__ double2 tm[];
   const int K = 2 * nsl2;
-  double2* sM = tm;          // [K][K]
-  double2* sR = tm + K * K;  // [K][TMUL_I]
+  double2* sM = tm;                              // [8 MF][MS], zero beyond K x K
+  double2* sR = tm + 8 * TMUL_MF * TMUL_MS;  // [KP][RS], zero beyond K
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nch = (npad + TMUL_I - 1) / TMUL_I, nitem = nch * ndf;
   const int it0 = blockIdx.x * per, it1 = min(nitem, it0 + per);
+  for (int idx = tid; idx < 8 * TMUL_MF * TMUL_MS + TMUL_KP * TMUL_RS; idx += 32 * TMUL_WARPS) tm[idx] = cmk(0.0, 0.0);
   int staged = -1;
   for (int item = it0; item < it1; item++) {
     const int a = item / nch, i0 = (item % nch) * TMUL_I;
-    __syncthreads();  // the previous item's smem reads are done
+    __syncthreads();  // the previous item's smem reads (or the zero fill) are done
     if (a != staged) {
       const double2* T = tns + (size_t)atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2;
       for (int idx = tid; idx < K * K; idx += 32 * TMUL_WARPS) {
         const int row = idx / K, col = idx % K;
         const int ro = row / nsl2, la = row % nsl2, r = col / nsl2, b = col % nsl2;
         const int blk = ro == 0 ? (r == 0 ? 0 : 1) : (r == 0 ? 3 : 4);  // TUU TDU / TUD TDD
-        l1g_cp16(&sM[idx], &T[((size_t)blk * L1G_NSL2 + la) * L1G_NSL2 + b]);
+        l1g_cp16(&sM[row * TMUL_MS + col], &T[((size_t)blk * L1G_NSL2 + la) * L1G_NSL2 + b]);
       }
       staged = a;
     }
     const double2* R = Rop + (size_t)a * K * npad;
     for (int idx = tid; idx < K * TMUL_I; idx += 32 * TMUL_WARPS) {
-      const int k = idx / TMUL_I, c = idx % TMUL_I;
-      if (i0 + c < npad)
-        l1g_cp16(&sR[idx], &R[(size_t)k * npad + i0 + c]);
-      else
-        sR[idx] = make_double2(0.0, 0.0);
+      const int k = idx / TMUL_I, c = idx % TMUL_I;  // npad is a multiple of 64
+      l1g_cp16(&sR[k * TMUL_RS + c], &R[(size_t)k * npad + i0 + c]);
     }
     l1g_cp_wait_all();
     __syncthreads();
-    const int r0 = w * TMUL_ROWS;
-    if (r0 < K) {  // warp-uniform
-      double2 acc[TMUL_ROWS][2];
+    double re[TMUL_MF][2][2], im[TMUL_MF][2][2];
 #pragma unroll
-      for (int r = 0; r < TMUL_ROWS; r++) acc[r][0] = acc[r][1] = cmk(0.0, 0.0);
-#pragma unroll 2
-      for (int k = 0; k < K; k++) {
-        const double2 x0 = sR[k * TMUL_I + lane], x1 = sR[k * TMUL_I + lane + 32];
+    for (int u = 0; u < TMUL_MF; u++)
 #pragma unroll
-        for (int r = 0; r < TMUL_ROWS; r++) {
-          const double2 m = sM[min(r0 + r, K - 1) * K + k];  // rows past K: computed, not stored
-          acc[r][0].x = fma(m.x, x0.x, fma(m.y, x0.y, acc[r][0].x));
-          acc[r][0].y = fma(m.y, x0.x, fma(-m.x, x0.y, acc[r][0].y));
-          acc[r][1].x = fma(m.x, x1.x, fma(m.y, x1.y, acc[r][1].x));
-          acc[r][1].y = fma(m.y, x1.x, fma(-m.x, x1.y, acc[r][1].y));
+      for (int v = 0; v < 2; v++) re[u][v][0] = re[u][v][1] = im[u][v][0] = im[u][v][1] = 0.0;
+    const double2* pM = sM + (lane >> 2) * TMUL_MS + (lane & 3);
+    const double2* pR = sR + (lane & 3) * TMUL_RS + 16 * w + (lane >> 2);
+    for (int k = 0; k < K; k += 4) {
+      double2 m[TMUL_MF], x[2];
+#pragma unroll
+      for (int v = 0; v < 2; v++) x[v] = pR[k * TMUL_RS + 8 * v];
+#pragma unroll
+      for (int u = 0; u < TMUL_MF; u++) m[u] = pM[8 * u * TMUL_MS + k];
+      // m conj(x)
+#pragma unroll
+      for (int u = 0; u < TMUL_MF; u++)
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          dmma(re[u][v], m[u].x, x[v].x);
+          dmma(im[u][v], m[u].y, x[v].x);
         }
-      }
-      double2* L = Lop + (size_t)a * K * npad;
 #pragma unroll
-      for (int r = 0; r < TMUL_ROWS; r++) {
-        const int row = r0 + r;
-        if (row < K) {
-          if (i0 + lane < npad) L[(size_t)row * npad + i0 + lane] = acc[r][0];
-          if (i0 + lane + 32 < npad) L[(size_t)row * npad + i0 + lane + 32] = acc[r][1];
+      for (int u = 0; u < TMUL_MF; u++)
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          dmma(re[u][v], m[u].y, x[v].y);
+          dmma(im[u][v], -m[u].x, x[v].y);
         }
-      }
+    }
+    double2* L = Lop + (size_t)a * K * npad + i0 + 16 * w + 2 * (lane & 3);
+#pragma unroll
+    for (int u = 0; u < TMUL_MF; u++) {
+      const int row = 8 * u + (lane >> 2);
+      if (row < K)
+#pragma unroll
+        for (int v = 0; v < 2; v++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) L[(size_t)row * npad + 8 * v + e] = cmk(re[u][v][e], im[u][v][e]);
     }
   }
 }
@@ -895,11 +917,6 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
 #define TRI_THREADS 128
 __host__ __device__ constexpr int tri_smem_bytes(int wt) { return TRI_STAGES * 2 * TRI_KC * (2 * wt + 2) * 16; }
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
 // 16-byte copy, or zeros when !in (src is not read then)
 __device__ __forceinline__ void l1g_cp16z(void* dst, const void* src, bool in) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);

@@ -1,0 +1,114 @@
+"""Edges of the kernels' tiles and branches, against the oracle or the FP64
+path: row counts around the tile sizes, every l count, orbital l of 0..3,
+projection slices, bands and row blocks that fill no tile."""
+import numpy as np
+import pytest
+import torch
+
+from hack_wein2k_b200 import lapw1gpu, synth
+from oracle import oracle as O
+from tests.helpers import rel_errors
+
+TOL_FP64 = 1e-12
+# the slice counts' bounds of tests/test_split_gpu.py
+TOL_SPLIT = {4: 2e-7, 5: 2e-9, 6: 2e-11, 7: 1e-12}
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(p, nv):
+    """The problem's first nv plane waves (no local orbitals)."""
+    assert p.nlo == 0 and nv <= p.nv
+    return p.copy(nv=nv, kzz=p.kzz[:nv], xk=p.xk[:nv], yk=p.yk[:nv], zk=p.zk[:nv], rk=p.rk[:nv])
+
+
+def _plain(rkmax, k=(0.13, 0.27, 0.41), lmax=10, **kw):
+    return synth.synth_problem(synth.cell_small_mixed(), rkmax, k, seed=11, lmax=lmax, **kw)
+
+
+def _check(ctx, p, tol):
+    hs, hsd = ctx.setup(p)
+    err = rel_errors(hs, hsd, *O.setup(p))
+    assert err["H"] <= tol and err["S"] <= tol, (p.n, err)
+
+
+# 32- and 64-row tiles of k_spherical and k_tri_gemm; 1537 rows take the
+# 64-wide product tiles (300 of them), 1472 the 32-wide ones
+@pytest.mark.parametrize("nv", [1, 31, 32, 33, 63, 64, 65, 97, 1472, 1537])
+def test_fp64_row_counts(ctx, nv):
+    ctx.set_precision(lapw1gpu.PREC_FP64)
+    _check(ctx, _rows(_plain(6.0 if nv < 200 else 13.5), nv), TOL_FP64)
+
+
+@pytest.mark.parametrize("lmax", [4, 9, 10, 12])
+@pytest.mark.parametrize("lnsmax", [0, 2, 4])
+def test_fp64_l_counts(ctx, lmax, lnsmax):
+    """k_spherical with fewer and more l than its unrolled count, the HNS
+    operand product with 2, 18 and 50 rows, LO rows on every atom."""
+    ctx.set_precision(lapw1gpu.PREC_FP64)
+    _check(ctx, _plain(5.0, lmax=lmax, lnsmax=lnsmax, lo_l=(0, 1, 2), rotate_local=True), TOL_FP64)
+
+
+@pytest.mark.parametrize("slices", [4, 5, 6, 7])
+@pytest.mark.parametrize("lmax", [4, 10, 12])
+def test_split_row_counts(ctx, slices, lmax):
+    """k_sph_tc at the edges of its 12- and 8-I and 128-J tiles: an element
+    depends on its two rows only (scales are per row, the level sums exact), so
+    the first nv rows alone give the bits they have in the whole problem,
+    which is within the slices' bound of the oracle.  k along an axis puts many
+    pairs on one line (the x P_(l-1) branch)."""
+    full = _plain(6.0, k=(0.0, 0.0, 0.3), lmax=lmax)
+    ctx.set_precision(lapw1gpu.PREC_SPLIT, slices)
+    try:
+        hs, hsd = ctx.setup(full, stages=1)
+        err = rel_errors(hs, hsd, *O.setup(full, stages=1))
+        assert err["H"] <= TOL_SPLIT[slices] and err["S"] <= TOL_SPLIT[slices], err
+        for nv in (1, 7, 8, 9, 11, 12, 13, 127, 128, 129):
+            h, d = ctx.setup(_rows(full, nv), stages=1)
+            assert np.array_equal(h, hs[:nv, :nv]) and np.array_equal(d, hsd[:nv]), nv
+    finally:
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+
+
+@pytest.mark.parametrize("prec,tol", [(lapw1gpu.PREC_FP64, TOL_FP64), (lapw1gpu.PREC_SPLIT, TOL_SPLIT[7])])
+@pytest.mark.parametrize("orb", [((1, (0,)),), ((1, (3, 1)), (2, (0, 2, 3)))])
+def test_orbital_l(ctx, prec, tol, orb):
+    ctx.set_precision(prec, 7)
+    try:
+        _check(ctx, _plain(5.0, lo_l=(0, 2), apw_l=(1,), rotate_local=True, orb=orb), tol)
+    finally:
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+
+
+# bands around a tile of 40 (32 at 7 and 8 slices), blocks whose last rows
+# fill no K block of 64
+@pytest.mark.parametrize("slices,nb,block,lmax", [(4, 40, 64, 10), (5, 1, 96, 8), (6, 41, 64, 12), (6, 39, 160, 10),
+                                                  (7, 33, 64, 9), (8, 31, 128, 10)])
+def test_projection_tiles(ctx, slices, nb, block, lmax):
+    """The projections against the FP64 adjoint of the same vectors.  The
+    slices leave (S+1) 2^(-7S) of the largest terms, whose sum over some
+    hundred rows exceeds the result by less than 64; 1e-9 for pairs that the
+    pair kernel takes as parallel."""
+    p = _plain(7.0, lmax=lmax, lo_l=(0, 1), rotate_local=True)
+    assert p.nv > 2 * block
+    rng = np.random.default_rng(5)
+    dev = torch.device("cuda", ctx.device)
+    c = torch.from_numpy(rng.standard_normal((nb, p.n)) + 1j * rng.standard_normal((nb, p.n))).to(dev)
+    eps = torch.from_numpy(np.sort(rng.uniform(-1.0, 1.0, nb))).to(dev)
+    occ = torch.from_numpy(rng.uniform(0.0, 2.0, nb)).to(dev)
+    kp = ctx.upload(p)
+    out = []
+    try:
+        for prec in (lapw1gpu.PREC_FP64, lapw1gpu.PREC_SPLIT):
+            ctx.set_precision(prec, 7)
+            ctx.set_force_slices(8, 8)
+            ctx.set_force_projection(slices, block)
+            g = torch.empty((p.ndf, 3), dtype=torch.float64, device=dev)
+            kp.forces(c.data_ptr(), p.n, nb, occ.data_ptr(), eps.data_ptr(), g.data_ptr())
+            out.append(g.cpu().numpy())
+    finally:
+        kp.free()
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+        ctx.set_force_slices(6, 6)
+        ctx.set_force_projection(-1, 1024)
+    assert np.abs(out[1] - out[0]).max() <= (64 * (slices + 1) * 2.0 ** (-7 * slices) + 1e-9) * np.abs(out[0]).max()
