@@ -826,13 +826,11 @@ __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int n
 
 // LO rows: A2 += TUU21 conj(CLM), B2 += TUD21 conj(CLM),
 // C2 = TUU12 conj(ALM) + TDU12 conj(BLM) + TUU22 conj(CLM)  (hns.F:391-433).
-// One thread per (la, 4 LO rows) of an atom: block (32 la, 8) over 32 rows,
-// the rows' ALM, BLM, CLM staged in shared memory; each T element read is
-// used for the 4 rows.
-// An LO row has ALM, BLM, CLM on the atoms of its own type only: a block
-// whose rows are all zero on the atom writes C2 = 0 and leaves L as it is (39
-// of 40 blocks at 40 types); the T elements of 5 b are loaded together (one b
-// at a time each waited for its own, 27 us for 72 rows).
+// Block (32 la, 8) over 32 LO rows of an atom: a warp takes 4 of them in turn,
+// lane la.  A row has ALM, BLM, CLM on the atoms of its own type only, and
+// there only at its own l: the sums run over the non-zero b (bits of a ballot;
+// NaN counts as non-zero), 1 + 3 + 5 of 25 for s, p and d rows, and a row
+// that is zero on the atom writes C2 = 0 and leaves L as it is.
 #define LOOPS_ROWS 32
 __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __restrict__ tns,
                                                     double2* __restrict__ Lop, const double2* __restrict__ Rop,
@@ -843,7 +841,6 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
   const int a = blockIdx.y;
   const int nsl2 = (P.lnsmax + 1) * (P.lnsmax + 1);
   const size_t npad = P.npad;
-  bool some = false;  // a non-zero (or NaN) coefficient of the block's rows on this atom
   for (int q = threadIdx.y * 32 + threadIdx.x; q < LOOPS_ROWS * 3 * nsl2; q += 256) {
     const int r = q / (3 * nsl2), w = (q / nsl2) % 3, b = q % nsl2;
     const int cc = c0 + r;
@@ -856,46 +853,40 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
         v = Clo[((size_t)a * nsl2 + b) * P.nlo + cc];
     }
     sX[r][w][b] = v;
-    some |= v.x != 0.0 || v.y != 0.0;
   }
-  if (!__syncthreads_or(some)) {
-    if (la < nsl2)
-      for (int c = c0 + cy; c < min(P.nlo, c0 + LOOPS_ROWS); c += 8)
-        C2lo[((size_t)a * nsl2 + la) * P.nlo + c] = cmk(0.0, 0.0);
-    return;
-  }
-  if (la >= nsl2 || c0 + cy >= P.nlo) return;
-  const double2* T = tns + (size_t)P.atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2;
-  double2 da[4], db[4], dc[4];
-#pragma unroll
-  for (int u = 0; u < 4; u++) da[u] = db[u] = dc[u] = cmk(0, 0);
-#pragma unroll 5
-  for (int b = 0; b < nsl2; b++) {
-#define TT(blk) __ldg(T + ((size_t)(blk)*L1G_NSL2 + la) * L1G_NSL2 + b)
-    const double2 tuu21 = TT(2), tud21 = TT(5), tuu12 = TT(6), tdu12 = TT(7), tuu22 = TT(8);
-#undef TT
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int r = cy + 8 * u;
-      const double2 A = sX[r][0][b], B = sX[r][1][b], Cc = sX[r][2][b];
-      da[u] = cadd(da[u], cmul(tuu21, cconj(Cc)));
-      db[u] = cadd(db[u], cmul(tud21, cconj(Cc)));
-      dc[u] = cadd(dc[u], cadd(cadd(cmul(tuu12, cconj(A)), cmul(tdu12, cconj(B))), cmul(tuu22, cconj(Cc))));
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const int c = c0 + cy + 8 * u;
+  __syncthreads();
+  const double2* T = tns + (size_t)P.atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2 + min(la, nsl2 - 1) * L1G_NSL2;
+  for (int u = 0; u < LOOPS_ROWS / 8; u++) {
+    const int r = cy + 8 * u, c = c0 + r;  // warp-uniform
     if (c >= P.nlo) break;
-    const size_t i = P.nv + c;
-    double2* LA = Lop + ((size_t)(a * 2 + 0) * nsl2 + la) * npad + i;
-    double2* LB = Lop + ((size_t)(a * 2 + 1) * nsl2 + la) * npad + i;
-    *LA = cadd(*LA, da[u]);
-    *LB = cadd(*LB, db[u]);
-    C2lo[((size_t)a * nsl2 + la) * P.nlo + c] = dc[u];
+    bool nz = false;
+    if (la < nsl2)
+#pragma unroll
+      for (int w = 0; w < 3; w++) nz |= sX[r][w][la].x != 0.0 || sX[r][w][la].y != 0.0;
+    unsigned bits = __ballot_sync(0xffffffffu, nz);
+    if (la >= nsl2) continue;
+    double2 da = cmk(0, 0), db = da, dc = da;
+    const bool some = bits != 0;
+    for (; bits; bits &= bits - 1) {
+      const int b = __ffs(bits) - 1;
+      const double2 A = cconj(sX[r][0][b]), B = cconj(sX[r][1][b]), Cc = cconj(sX[r][2][b]);
+#define TT(blk) __ldg(T + (size_t)(blk)*L1G_NSL2 * L1G_NSL2 + b)
+      const double2 tuu21 = TT(2), tud21 = TT(5), tuu12 = TT(6), tdu12 = TT(7), tuu22 = TT(8);
+#undef TT
+      da = cadd(da, cmul(tuu21, Cc));
+      db = cadd(db, cmul(tud21, Cc));
+      dc = cadd(dc, cadd(cadd(cmul(tuu12, A), cmul(tdu12, B)), cmul(tuu22, Cc)));
+    }
+    if (some) {
+      const size_t i = P.nv + c;
+      double2* LA = Lop + ((size_t)(a * 2 + 0) * nsl2 + la) * npad + i;
+      double2* LB = Lop + ((size_t)(a * 2 + 1) * nsl2 + la) * npad + i;
+      *LA = cadd(*LA, da);
+      *LB = cadd(*LB, db);
+    }
+    C2lo[((size_t)a * nsl2 + la) * P.nlo + c] = dc;
   }
 }
-
 
 // ---------------------------------------------------------------------
 // out(i,j) (+)= sum_k L[k][i] R[k][j] on the lower triangle i >= j, i, j < n
