@@ -125,6 +125,9 @@ struct lapw1gpu_context {
   int sph_tc = 1;          // split precision: spherical part on tcgen05 (1) or FP64 (0)
   int sph_kb = 128;        // k_sph_tc: bytes of K per pipeline stage (64: deep ring, 128: two stages)
   int batch_sets = 2;      // concurrent k-point chains in a batch
+  // chosen by the caller or the autotuner; until then a rule on the sizes
+  // decides (sph_kb128, batch_chains)
+  bool sph_kb_set = false, batch_sets_set = false;
   int test_never_wait = 0; // test hook: the spherical tensor kernel's consumer wait runs out
   int last_launches = 0;   // kernels launched by the last call (a library product counts as one)
   std::map<std::string, DevBuf> bufs;
@@ -1038,13 +1041,23 @@ static int sph_level_mode(int S, int Kp) {
 // true when the split-precision spherical path handles this slice count
 static bool sph_tc_supported(int S) { return S >= 4 && S <= 7; }
 
+// 128-byte K blocks in k_sph_tc, for K = Kp bytes per row?  They fit two stages
+// up to 5 slices.  Where no value was chosen: 64-byte blocks when they pad K
+// less (the rest of the last block is fed as zeros): K = 160 1.37 ms against
+// 1.44 (40 atoms), K = 416 21.1 against 23.0 (100 atoms); at equal padding the
+// halved count of blocks is up to 2.5% faster (K = 256: 1.59 against 1.62).
+static bool sph_kb128(const lapw1gpu_context* c, int Kp) {
+  if (c->slices > 5) return false;
+  if (c->sph_kb_set) return c->sph_kb == 128;
+  return (Kp + 63) / 64 * 64 == (Kp + 127) / 128 * 128;
+}
+
 static int sph_tc_dispatch(lapw1gpu_context* c, lapw1gpu_kpoint* k, int set, const DevProb& P, const SphCoef* coef,
                            const double2* tab, double2* hs, int ld, double2* hsdiag, cudaStream_t s, int* nl,
                            const cudaEvent_t* ev, HnsPipe* sp) {
   const int Kp = 2 * round_up(2 * k->ndf, 16);
   const int mode = sph_level_mode(c->slices, Kp);
-  // 128-byte K blocks fit two stages up to 5 slices
-  const bool kb128 = c->sph_kb == 128 && c->slices <= 5;
+  const bool kb128 = sph_kb128(c, Kp);
 #define SPH_MODES(SS, KB)                                                                             \
   return mode == 2   ? sph_tc_launch<SS, 2, KB>(c, k, set, P, coef, tab, hs, ld, hsdiag, s, nl, ev, sp) \
          : mode == 1 ? sph_tc_launch<SS, 1, KB>(c, k, set, P, coef, tab, hs, ld, hsdiag, s, nl, ev, sp) \
@@ -1355,9 +1368,21 @@ int lapw1gpu_kpoint_run(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, dou
 }
 
 // ---- k-point batches: one captured graph per argument set ----
+// Concurrent chains of a batch where the caller chose none: a k-point of up
+// to L1G_SMALL_N rows leaves most SMs idle in most of its kernels (fewer than
+// four 32 x 32 pair tiles per SM), so its batch runs on every chain there is (16
+// k-points of N = 704, FP64: 1.10 ms on four chains, 1.59 on two); larger ones on
+// two (four k-points of N = 4950: kernels that fill the SMs anyway).
+#define L1G_SMALL_N 1088
+static int batch_chains(const lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int nk) {
+  if (c->batch_sets_set) return std::max(1, std::min(c->batch_sets, L1G_MAX_SETS));
+  int n = 0;
+  for (int i = 0; i < nk; i++) n = std::max(n, kps[i]->n);
+  return n <= L1G_SMALL_N ? L1G_MAX_SETS : 2;
+}
 static int batch_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int nk, int stages, double* const* d_hs,
                          const int* ldhs, double* const* d_hsdiag, int* nl) {
-  const int sets = std::max(1, std::min(c->batch_sets, L1G_MAX_SETS));
+  const int sets = batch_chains(c, kps, nk);
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
   CK(cudaEventRecord(c->fork, c->stream));
   for (int q = 1; q < sets; q++) CK(cudaStreamWaitEvent(c->side[q], c->fork, 0));
@@ -1384,7 +1409,8 @@ int lapw1gpu_setup_batch(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int n
   std::vector<uintptr_t> key = {(uintptr_t)nk,         (uintptr_t)stages,        (uintptr_t)c->prec,
                                 (uintptr_t)(c->slices * 16 + c->slices_hns), (uintptr_t)c->hns_diag_b,
                                 (uintptr_t)c->split_group,
-                                (uintptr_t)c->sph_tc,  (uintptr_t)c->sph_kb, (uintptr_t)c->batch_sets,
+                                (uintptr_t)c->sph_tc,  (uintptr_t)(c->sph_kb * 2 + c->sph_kb_set),
+                                (uintptr_t)batch_chains(c, kps, nk),
                                 (uintptr_t)c->test_never_wait};
   for (int i = 0; i < nk; i++) {
     key.push_back((uintptr_t)kps[i]);
@@ -1473,6 +1499,10 @@ int lapw1gpu_set_tuning(lapw1gpu_context* c, const lapw1gpu_tuning* t) {
   c->hns_diag_b = t->hns_diag_b;
   c->split_group = t->split_group;
   c->sph_tc = t->sph_tc;
+  // (a value that is reported already is not a choice: callers that change
+  // one field write the others back)
+  if (t->batch_sets != c->batch_sets) c->batch_sets_set = true;
+  if (t->sph_kblock != c->sph_kb) c->sph_kb_set = true;
   c->batch_sets = t->batch_sets;
   c->sph_kb = t->sph_kblock;
   return LAPW1GPU_OK;
@@ -1521,7 +1551,11 @@ int lapw1gpu_autotune(lapw1gpu_context* c, lapw1gpu_kpoint* kp, double* d_hs, in
     if (sph_tc_supported(c->slices)) rc = tune(&c->sph_tc, {1, 0}, T_TOTAL);
     // the K block (and with it the ring depth) of k_sph_tc: 128-byte blocks
     // exist up to 5 slices
-    if (!rc && c->sph_tc && c->slices <= 5) rc = tune(&c->sph_kb, {64, 128}, T_SPH);
+    if (!rc && c->sph_tc && c->slices <= 5) {
+      if (!c->sph_kb_set) c->sph_kb = sph_kb128(c, 2 * round_up(2 * kp->ndf, 16)) ? 128 : 64;  // the value held
+      c->sph_kb_set = true;
+      rc = tune(&c->sph_kb, {64, 128}, T_SPH);
+    }
     if (!rc) rc = tune(&c->split_group, {4, 8, 16, 32}, T_HNS);
   }
   if (rc) return rc;
