@@ -458,143 +458,67 @@ __global__ void __launch_bounds__(FRC_THREADS) k_force_bins(DevProb P, const int
   }
 }
 
-// local-orbital columns: k_lo's terms per equivalent atom, reduced per warp
-__global__ void k_force_lo(DevProb P, const LoCol* __restrict__ cols, const double2* __restrict__ rho,
-                           const double2* __restrict__ rhoe, int ldr, int rt, double* __restrict__ F) {
-  const LoCol c = cols[blockIdx.y];
-  const int nv = P.nv;
-  const int I = nv + c.nnlo - 1;
-  if ((int)(blockIdx.x * blockDim.x) >= I) return;  // no pair J < I in the block (block-uniform)
-  const int J = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const int jn = c.jn, l = c.l, jlo = c.jlo, jeqo = c.jeqo, mo1 = c.mo1, mult = P.mult[jn];
-  const double pi = 3.141592653589793238462643;
-  const double r = P.rmt[jn], r2 = r * r;
-  const double pi4r2v = 4.0 * pi * sqrt(P.vi) * r * r;
-  const int o = jn * P.ldl + l;
-  const double U = P.p[o], UP = P.pe[o], DU = P.dp[o], DUP = P.dpe[o], CHN = P.pei[o], E = P.e[o];
-  const int lo4 = jn * (L1G_LOMAX + 1) + l;
-#define LOV(arr, jj) P.arr[(jn * L1G_NLOAT + (jj)-1) * (L1G_LOMAX + 1) + l]
-  const double ALO = LOV(alo, jlo), BLO = LOV(blo, jlo), CLO = LOV(clo, jlo), ELO = LOV(elo, jlo);
-  const double PI12 = P.pi12lo[lo4], PE12 = P.pe12lo[lo4], DPL = P.dplo[lo4];
-  const double c1r = ALO + PI12 * CLO;
-  const double c2r = BLO * CHN + PE12 * CLO;
-  const double c11r = ALO * E + 0.5 * (BLO + CLO * PI12 * (ELO + E));
-  const double c12r = BLO * CHN * E + 0.5 * (ALO + CLO * PI12 + CLO * PE12 * (ELO + E));
-  const double c3r = CLO + PE12 * BLO + ALO * PI12;
-  const double c13r = CLO * ELO + 0.5 * (BLO * PI12 + (ELO + E) * (ALO * PI12 + PE12 * BLO));
-  const double akinlor = 0.5 * r2 * (ALO * DU + BLO * DUP + CLO * DPL);
-  const double clr = c.clr, cli = c.cli;
-  bool inlo[L1G_NLOAT + 1];
-  const int Jf = J + 1;
-  bool any_lo = false;
-  for (int jlop = 1; jlop <= jlo; jlop++) {
-    int jbeg = nv + c.nnlo - (mo1 + l) - (2 * l + 1) * (jeqo - 1) - (jlo - jlop) * (2 * l + 1) * mult;
-    int jend = nv + c.nnlo - (jlo - jlop) * (mo1 + l + 1) - (jlo - jlop) * (jeqo - 1) * (2 * l + 1);
-    inlo[jlop] = (Jf >= jbeg && Jf <= jend);
-    any_lo |= inlo[jlop];
-  }
-  const bool act = (J < I) && (J < nv || any_lo);
-  double dxc[3] = {0.0, 0.0, 0.0};
-  double2 rj = cmk(0.0, 0.0), re = cmk(0.0, 0.0);
-  double alj = 0.0, blj = 0.0;
-  if (act) {
-    dxc[0] = FRC_2PI * (P.kzz[3 * I] - P.kzz[3 * J]);
-    dxc[1] = FRC_2PI * (P.kzz[3 * I + 1] - P.kzz[3 * J + 1]);
-    dxc[2] = FRC_2PI * (P.kzz[3 * I + 2] - P.kzz[3 * J + 2]);
-    rj = rt ? cconj(rho[(size_t)J * ldr + I]) : rho[(size_t)I * ldr + J];
-    re = rt ? cconj(rhoe[(size_t)J * ldr + I]) : rhoe[(size_t)I * ldr + J];
-    if (J < nv) {
-      size_t oo = ((size_t)jn * P.ltop + l) * P.nvpad + J;
-      alj = P.al[oo];
-      blj = P.bl[oo];
-    }
-  }
-  // the LO row's Y_lm per equivalent atom, shared by the block (I is the
-  // block's), in chunks of FRC_YCH atoms
-  constexpr int FRC_YCH = 16;
-  __shared__ double2 syi[FRC_YCH][16];
-  for (int jeq = 0; jeq < mult; jeq++) {
-    const int a = c.a0 + jeq;
-    if (jeq % FRC_YCH == 0) {  // block-uniform
+// local-orbital columns: k_lo's terms per equivalent atom and group of 2l+1
+// columns; one atomic per block, atom and component
+__global__ void __launch_bounds__(128) k_force_lo(DevProb P, const LoCol* __restrict__ cols,
+                                                  const int* __restrict__ groups, const double2* __restrict__ rho,
+                                                  const double2* __restrict__ rhoe, int ldr, int rt,
+                                                  double* __restrict__ F) {
+  __shared__ double2 sy[7][LO_YCH][7];
+  __shared__ double wsum[4][3];  // blockDim.x = 128: 4 warps
+  const LoCol c = cols[groups[blockIdx.y]];
+  const int nv = P.nv, nm = 2 * c.l + 1, I0 = nv + c.nnlo - 1, mult = P.mult[c.jn];
+  const int J = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  if ((int)(blockIdx.x * blockDim.x) >= I0 + nm - 1) return;  // no pair J < I in the block (block-uniform)
+  const LoRad rad = lo_radial(P, c);
+  const bool act = J < I0 + nm - 1;
+  const double2 fpw = J < nv ? lo_pw_factors(P, c, rad, J) : cmk(0.0, 0.0);
+  const int k0 = act ? P.kzz[3 * J] : 0, k1 = act ? P.kzz[3 * J + 1] : 0, k2 = act ? P.kzz[3 * J + 2] : 0;
+  for (int e = 0; e < mult; e++) {
+    const int a = c.a0 + e;
+    if (e % LO_YCH == 0) {  // block-uniform
       __syncthreads();
-      const int q = threadIdx.x;
-      if (q < FRC_YCH && jeq + q < mult)
-        dev_ylm_row<3>(P.xk[I], P.yk[I], P.zk[I], P.rotij + 9 * (a + q), P.rotloc + 9 * jn, l, syi[q]);
+      lo_stage_y(P, c, e, sy);
       __syncthreads();
     }
-    double2 S = cmk(0.0, 0.0), H = cmk(0.0, 0.0);
+    double f0 = 0.0, f1 = 0.0, f2 = 0.0;
     if (act) {
-      const double* ra = P.pos + 3 * a;
-      double s = ra[0] * (double)(P.kzz[3 * I] - P.kzz[3 * J]) + ra[1] * (double)(P.kzz[3 * I + 1] - P.kzz[3 * J + 1]) +
-                 ra[2] * (double)(P.kzz[3 * I + 2] - P.kzz[3 * J + 2]);
-      const double2 ph = cconj(cexp2pi(s));
-      double2 yj[16];
-      const double2* yi = syi[jeq % FRC_YCH];
-      dev_ylm_row<3>(P.xk[J], P.yk[J], P.zk[J], P.rotij + 9 * a, P.rotloc + 9 * jn, l, yj);
-      for (int mo2 = -l; mo2 <= l; mo2++) {
-        const int lm = l * (l + 1) + mo2;
-        const double clylnr = clr * yi[lm].x + cli * yi[lm].y;
-        const double clylni = cli * yi[lm].x - clr * yi[lm].y;
-        const double c1rup = c1r * clylnr * pi4r2v, c1iup = c1r * clylni * pi4r2v;
-        const double c2rup = c2r * clylnr * pi4r2v, c2iup = c2r * clylni * pi4r2v;
-        const double c3rup = c3r * clylnr * pi4r2v, c3iup = c3r * clylni * pi4r2v;
-        const double c11rup = c11r * clylnr * pi4r2v, c11iup = c11r * clylni * pi4r2v;
-        const double c12rup = c12r * clylnr * pi4r2v, c12iup = c12r * clylni * pi4r2v;
-        const double c13rup = c13r * clylnr * pi4r2v, c13iup = c13r * clylni * pi4r2v;
-        const double akinlorup = akinlor * clylnr * pi4r2v, akinloiup = akinlor * clylni * pi4r2v;
-        const double clylr = clr * yj[lm].x + cli * yj[lm].y;
-        const double clyli = cli * yj[lm].x - clr * yj[lm].y;
-        if (J < nv) {
-          const double c6r = clylr * alj * pi4r2v, c6i = clyli * alj * pi4r2v;
-          const double c7r = clylr * blj * pi4r2v, c7i = clyli * blj * pi4r2v;
-          double cabr = c6r * c1rup + c7r * c2rup + c6i * c1iup + c7i * c2iup;
-          double cabi = -c6i * c1rup - c7i * c2rup + c6r * c1iup + c7r * c2iup;
-          S = cadd(S, cmk(cabr * ph.x - cabi * ph.y, cabr * ph.y + cabi * ph.x));
-          cabr = c6r * c11rup + c7r * c12rup + c6i * c11iup + c7i * c12iup;
-          cabi = -c6i * c11rup - c7i * c12rup + c6r * c11iup + c7r * c12iup;
-          const double ua = c6r * U + c7r * UP, ub = c6i * U + c7i * UP;
-          const double akinbr = ua * akinlorup + ub * akinloiup;
-          const double akinbi = ua * akinloiup - ub * akinlorup;
-          H = cadd(H, cmk(cabr * ph.x - cabi * ph.y, cabr * ph.y + cabi * ph.x));
-          H = cadd(H, cmk(akinbr * ph.x - akinbi * ph.y, akinbr * ph.y + akinbi * ph.x));
-        } else {
-          for (int jlop = 1; jlop <= jlo; jlop++) {
-            if (!inlo[jlop]) continue;
-            const double alop = LOV(alo, jlop), blop = LOV(blo, jlop), clop = LOV(clo, jlop);
-            const double c6r = clylr * alop * pi4r2v, c6i = clyli * alop * pi4r2v;
-            const double c7r = clylr * blop * pi4r2v, c7i = clyli * blop * pi4r2v;
-            const double c8r = clylr * clop * pi4r2v, c8i = clyli * clop * pi4r2v;
-            double cr = c6r * c1rup + c6i * c1iup + c7r * c2rup + c7i * c2iup + c8r * c3rup + c8i * c3iup;
-            double ci = -c6i * c1rup + c6r * c1iup - c7i * c2rup + c7r * c2iup - c8i * c3rup + c8r * c3iup;
-            S = cadd(S, cmk(cr * ph.x - ci * ph.y, cr * ph.y + ci * ph.x));
-            cr = c6r * c11rup + c6i * c11iup + c7r * c12rup + c7i * c12iup + c8r * c13rup + c8i * c13iup;
-            ci = -c6i * c11rup + c6r * c11iup - c7i * c12rup + c7r * c12iup - c8i * c13rup + c8r * c13iup;
-            H = cadd(H, cmk(cr * ph.x - ci * ph.y, cr * ph.y + ci * ph.x));
-          }
-        }
+      double2 v[7];
+      lo_row_y(P, c, J, a, v);
+#pragma unroll
+      for (int q = 0; q < 7; q++) {
+        const int I = I0 + q;
+        if (q >= nm || J >= I) continue;
+        const double2 f = J < nv ? fpw : lo_lo_factors(P, c, rad, J, q - c.l);
+        if (J >= nv && f.x == 0.0 && f.y == 0.0) continue;
+        const double2 t = lo_dot(P, nm, v, sy[q][e % LO_YCH], I, a);
+        const double2 rj = rt ? cconj(rho[(size_t)J * ldr + I]) : rho[(size_t)I * ldr + J];
+        const double2 re = rt ? cconj(rhoe[(size_t)J * ldr + I]) : rhoe[(size_t)I * ldr + J];
+        // HS(I,J) = H (lower), HS(J,I) = S (upper): h = conj(H), s = conj(S)
+        const double uim = f.y * (t.x * rj.y - t.y * rj.x);  // Im(conj(H) rho(J,I))
+        const double vim = f.x * (t.x * re.y - t.y * re.x);  // Im(conj(S) rhoE(J,I))
+        const double g = -2.0 * FRC_2PI * (uim - vim);
+        f0 = fma(g, (double)(P.kzz[3 * I] - k0), f0);
+        f1 = fma(g, (double)(P.kzz[3 * I + 1] - k1), f1);
+        f2 = fma(g, (double)(P.kzz[3 * I + 2] - k2), f2);
       }
     }
-    // HS(I,J) = H (lower), HS(J,I) = S (upper): h = conj(H), s = conj(S)
-    const double uim = H.x * rj.y - H.y * rj.x;  // Im(conj(H) rho(J,I))
-    const double vim = S.x * re.y - S.y * re.x;  // Im(conj(S) rhoE(J,I))
-    const double g = act ? -2.0 * (uim - vim) : 0.0;
-    // the block's sum (every block of a column belongs to one atom): warp
-    // sums, then one atomic per component and block
-    __shared__ double wsum[4][3];  // blockDim.x = 128: 4 warps
 #pragma unroll
-    for (int cc = 0; cc < 3; cc++) {
-      double v = g * dxc[cc];
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_down_sync(0xffffffffu, v, o2);
-      if (lane == 0) wsum[threadIdx.x >> 5][cc] = v;
+    for (int o = 16; o > 0; o >>= 1) {
+      f0 += __shfl_down_sync(0xffffffffu, f0, o);
+      f1 += __shfl_down_sync(0xffffffffu, f1, o);
+      f2 += __shfl_down_sync(0xffffffffu, f2, o);
+    }
+    if (lane == 0) {
+      wsum[threadIdx.x >> 5][0] = f0;
+      wsum[threadIdx.x >> 5][1] = f1;
+      wsum[threadIdx.x >> 5][2] = f2;
     }
     __syncthreads();
     if (threadIdx.x < 3) atomicAdd(&F[a * 3 + threadIdx.x], wsum[0][threadIdx.x] + wsum[1][threadIdx.x] +
                                                           wsum[2][threadIdx.x] + wsum[3][threadIdx.x]);
     __syncthreads();  // wsum is rewritten by the next equivalent atom
   }
-#undef LOV
 }
 
 // GC[g][b][i] = G_g(i) C(i, b): g = 0 the plain block, g = 1..3 the rows

@@ -211,6 +211,7 @@ struct lapw1gpu_kpoint {
   double vi = 0.0;
   TabDesc tab{};
   std::vector<LoCol> locols;
+  std::vector<int> logroups;  // first column (mo1 = -l) of each (type, l, jlo, jeqo)
   std::vector<LoRange> loranges;
   std::vector<int> mult, atype, afirst;
   // HORB description: its items (atom, l) and the products' K
@@ -225,6 +226,7 @@ struct lapw1gpu_kpoint {
   const double2* d_warp = nullptr;
   const double2* d_tns = nullptr;
   const LoCol* d_locols = nullptr;
+  const int* d_logroups = nullptr;
   const LoRange* d_loranges = nullptr;
   const double2* d_pots = nullptr;
   const OrbItem* d_orbs = nullptr;
@@ -612,7 +614,6 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   {
     int nnlo = 0;
     for (int jn = 0; jn < p->nat; jn++) {
-      double clr = 1.0, cli = 0.0;
       for (int l = 0; l <= L1G_LOMAX; l++) {
         int nil = p->ilo[jn * (L1G_LOMAX + 1) + l];
         for (int jlo = 1; jlo <= nil; jlo++) {
@@ -632,16 +633,12 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
               cc.mo1 = mo1;
               cc.nnlo = nnlo;
               cc.a0 = k->afirst[jn];
-              cc.clr = clr;
-              cc.cli = cli;
+              if (mo1 == -l) k->logroups.push_back((int)k->locols.size());
               k->locols.push_back(cc);
             }
           r.i2 = nnlo;
           k->loranges.push_back(r);
         }
-        double t = clr;
-        clr = -cli;
-        cli = t;
       }
     }
   }
@@ -717,6 +714,7 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   size_t ntns = (size_t)nat * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2;
   size_t o_tns = add(p->nohns ? nullptr : (const void*)p->tns, p->nohns ? 16 : sizeof(double2) * ntns);
   size_t o_locol = add(k->locols.data(), sizeof(LoCol) * k->locols.size());
+  size_t o_logr = add(k->logroups.data(), sizeof(int) * k->logroups.size());
   size_t o_lor = add(k->loranges.data(), sizeof(LoRange) * k->loranges.size());
   size_t o_pots = add(k->pots.data(), sizeof(double2) * k->pots.size());
   size_t o_orbs = add(k->orbs.data(), sizeof(OrbItem) * k->orbs.size());
@@ -832,6 +830,7 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
   k->d_warp = SEGP(const double2*, o_warp);
   k->d_tns = SEGP(const double2*, o_tns);
   k->d_locols = SEGP(const LoCol*, o_locol);
+  k->d_logroups = SEGP(const int*, o_logr);
   k->d_loranges = SEGP(const LoRange*, o_lor);
   k->d_pots = SEGP(const double2*, o_pots);
   k->d_orbs = SEGP(const OrbItem*, o_orbs);
@@ -1221,7 +1220,8 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     // ---- K-b': local-orbital columns ----
     if (k->nlo > 0) {
       nl++;
-      k_lo<<<dim3((n + 127) / 128, k->nlo), 128, 0, s>>>(P, k->d_locols, d_hs, ldhs, d_hsdiag, c->d_status);
+      k_lo<<<dim3((n + 127) / 128, (unsigned)k->logroups.size()), 128, 0, s>>>(P, k->d_locols, k->d_logroups, d_hs, ldhs,
+                                                                              d_hsdiag, c->d_status);
     }
     CK(cudaGetLastError());
     if (sp)  // groups whose columns reach the LO columns are final after k_lo
@@ -2110,7 +2110,8 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
                                                                                                           bins, d_grad);
   CK(cudaGetLastError());
   if (nlo > 0) {
-    k_force_lo<<<dim3((n + 127) / 128, nlo), 128, 0, s>>>(P, k->d_locols, rho, rhoe, n, rt, d_grad);
+    k_force_lo<<<dim3((n + 127) / 128, (unsigned)k->logroups.size()), 128, 0, s>>>(P, k->d_locols, k->d_logroups, rho,
+                                                                                 rhoe, n, rt, d_grad);
     nlf++;
   }
   if (timed) CK(cudaEventRecord(c->fev[4], s));
