@@ -109,6 +109,7 @@ struct lapw1gpu_context {
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
   cudaEvent_t stage_done = nullptr;
+  cudaEvent_t hamilt_done = nullptr;  // a host setup's HAMILT, for the copy stream
   int prec = LAPW1GPU_PREC_FP64;
   int slices = 5;      // int8 slices of the spherical part (split precision)
   int slices_hns = 5;  // int8 slices of the HNS update
@@ -396,6 +397,7 @@ int lapw1gpu_init(int device, lapw1gpu_context** out) {
   }
   cudaEventCreateWithFlags(&c->async_done, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&c->stage_done, cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&c->hamilt_done, cudaEventDisableTiming);
   // status words read back through mapped host memory (a one-thread kernel
   // stores them), not by copies, which would queue behind a running
   // lapw1gpu_setup_async's HS copies on the copy engines
@@ -442,6 +444,7 @@ int lapw1gpu_finalize(lapw1gpu_context* c) {
   if (c->h_status) cudaFreeHost(c->h_status);
   if (c->async_done) cudaEventDestroy(c->async_done);
   if (c->stage_done) cudaEventDestroy(c->stage_done);
+  if (c->hamilt_done) cudaEventDestroy(c->hamilt_done);
   if (c->h_stage) cudaFreeHost(c->h_stage);
   if (c->d_status) cudaFree(c->d_status);
   for (auto& e : c->ev) cudaEventDestroy(e);
@@ -1090,12 +1093,14 @@ static double alg_flops(const lapw1gpu_kpoint* k) {
 }
 
 // The stage sequence of one k-point on stream s with scratch set `set`.
-// ev: events to record between stages (null in a batch).  Host-side work
+// ev: events to record between stages (null where nobody asks for timings: a
+// record per kernel costs the host and the stream about 2 us each).
+// hamilt_done: recorded after HAMILT.  Host-side work
 // is limited to launches: every buffer and tile list already exists when
 // the same k-point ran once before, so the sequence can be captured.
 static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, double2* d_hs, int ldhs,
                            double2* d_hsdiag, cudaStream_t s, int set, const cudaEvent_t* ev, int* nlaunch,
-                           HnsPipe* hp = nullptr) {
+                           HnsPipe* hp = nullptr, cudaEvent_t hamilt_done = nullptr) {
   DevProb P = k->P;
   const int n = k->n, nv = k->nv, ltop = k->ltop, ndf = k->ndf, nat = k->nat;
   P.al = (double*)c->sbuf(set, "al", sizeof(double) * (size_t)nat * ltop * k->nvpad);
@@ -1231,6 +1236,7 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
           sp->srec[g] = true;
         }
     if (ev) CK(cudaEventRecord(ev[3], s));
+    if (hamilt_done) CK(cudaEventRecord(hamilt_done, s));
   } else if (ev) {
     CK(cudaEventRecord(ev[2], s));
     CK(cudaEventRecord(ev[3], s));
@@ -1619,7 +1625,8 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
   double2* hsdiag = reinterpret_cast<double2*>(hsdiag_);
   cudaEvent_t e0 = c->ev[7], e1 = c->ev[8], e2 = c->ev[9], e3 = c->ev[10], ecp = c->ev[11];
   cudaStream_t s = c->stream, cs = c->side[1];
-  CK(cudaEventRecord(e0, s));
+  const bool timed = st || async;  // (the timings of an asynchronous setup are asked for later)
+  if (timed) CK(cudaEventRecord(e0, s));
   lapw1gpu_kpoint* k = nullptr;
   int rc = kpoint_upload_impl(c, p, &k, true);
   if (rc) return rc;
@@ -1636,7 +1643,7 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
     cudaMemcpy2DAsync(d_hs, z * n, hs, z * ldhs, z * n, n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(d_hd, hsdiag, z * n, cudaMemcpyHostToDevice, s);
   }
-  CK(cudaEventRecord(e1, s));
+  if (timed) CK(cudaEventRecord(e1, s));
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(int), s));
   int nl = 0;
   const bool overlap = (stages & 1) && (stages & 6);
@@ -1671,10 +1678,11 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
     hp.ev[g] = c->hns_ev[g];
     hp.sev[g] = c->sph_ev[g];
   }
-  rc = kpoint_run_impl(c, k, stages, d_hs, n, d_hd, s, 0, c->ev, &nl, pipe ? &hp : nullptr);
+  rc = kpoint_run_impl(c, k, stages, d_hs, n, d_hd, s, 0, timed ? c->ev : nullptr, &nl, pipe ? &hp : nullptr,
+                       overlap ? c->hamilt_done : nullptr);
   c->last_launches = nl;
   if (rc == LAPW1GPU_OK) {
-    CK(cudaEventRecord(e2, s));
+    if (timed) CK(cudaEventRecord(e2, s));
     bool grouped = pipe && hp.groups > 0 && hp.col[hp.groups] == n;
     for (int g = 0; grouped && g < hp.groups; g++) grouped = hp.recorded[g] && hp.srec[g];
     if (grouped) {
@@ -1689,7 +1697,7 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
                               cudaMemcpyDeviceToHost, cs) != cudaSuccess)
           rc = LAPW1GPU_ERR_CUDA;
       }
-      CK(cudaStreamWaitEvent(cs, c->ev[3], 0));
+      CK(cudaStreamWaitEvent(cs, c->hamilt_done, 0));
       if (cudaMemcpyAsync(hsdiag, d_hd, z * n, cudaMemcpyDeviceToHost, cs) != cudaSuccess) rc = LAPW1GPU_ERR_CUDA;
       for (int g = 0; g < hp.groups; g++) {
         const int a = hp.col[g], w = hp.col[g + 1] - a;
@@ -1702,8 +1710,7 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
       CK(cudaEventRecord(ecp, cs));
       if (!async) CK(cudaStreamWaitEvent(s, ecp, 0));
     } else if (overlap) {
-      // c->ev[3] marks the end of HAMILT (+ LO columns) on s
-      CK(cudaStreamWaitEvent(cs, c->ev[3], 0));
+      CK(cudaStreamWaitEvent(cs, c->hamilt_done, 0));
       for (int c0 = L1G_D2H_PANEL; c0 < n; c0 += L1G_D2H_PANEL) {
         const int w = std::min(L1G_D2H_PANEL, n - c0);
         if (cudaMemcpy2DAsync(hs + (size_t)c0 * ldhs, z * ldhs, d_hs + (size_t)c0 * n, z * n, z * c0, w,
@@ -1740,7 +1747,7 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
       return LAPW1GPU_OK;
     }
   }
-  CK(cudaEventRecord(e3, s));
+  if (timed) CK(cudaEventRecord(e3, s));
   int hstat = 0;
   if (read_status(c, s, &hstat, &nl) != LAPW1GPU_OK) rc = rc ? rc : LAPW1GPU_ERR_CUDA;
   c->last_launches = nl;

@@ -235,10 +235,10 @@ class Context:
             hsdiag = np.zeros(n, dtype=np.complex128)
         assert hs.flags.f_contiguous and hs.dtype == np.complex128 and hs.shape[0] >= n
         cp = prob.to_c()
-        st = CStats()
+        st = CStats() if stats else None
         rc = self.lib.lapw1gpu_setup_stages(self.h, C.byref(cp), stages,
                                             _dp(hs.reshape(-1, order="F").view(np.float64)), hs.shape[0],
-                                            _dp(hsdiag.view(np.float64)), C.byref(st))
+                                            _dp(hsdiag.view(np.float64)), C.byref(st) if stats else None)
         _check("lapw1gpu_setup", rc)
         if stats:
             return hs, hsdiag, st.as_dict()
