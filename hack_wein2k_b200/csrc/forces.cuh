@@ -55,10 +55,9 @@ __host__ __device__ constexpr int frc_smem_bytes(int lt) {
 
 // One block per 32 x 32 pair tile, 256 threads.  Thread (warp, lane) owns
 // the 2 x 2 pairs J = j0 + jl0 + {0, 8}, I = i0 + il0 + {0, 4} with
-// jl0 = 16 (warp & 1) + (lane & 7), il0 = 8 (warp >> 1) + (lane >> 3):
+// jl0 = 16 (warp & 1) + pr_lane_j, il0 = 8 (warp >> 1) + pr_lane_i:
 // a warp reads 8 distinct J rows and 4 distinct I rows per l, so that the
-// shared-memory reads (about one cycle each: the addresses of a read are
-// 8 or 4 distinct 16-byte words) stay below the FP64 pipe's rate.  The
+// shared-memory reads (two cycles each) stay below the FP64 pipe's rate.  The
 // Legendre weights, rho, rhoE and dK of the four pairs stay in registers
 // for all types.  The type rows (k_pair_rows) and the phases of a chunk
 // are copied into shared memory by cp.async one chunk ahead (double
@@ -81,7 +80,7 @@ __global__ void __launch_bounds__(FRC_THREADS, 1)
   const int2 t = tiles[blockIdx.x];
   const int i0 = t.x * SPH_T, j0 = t.y * SPH_T;
   const int nv = P.nv, ltop = P.ltop, nat = P.nat, nvpad = P.nvpad;
-  const int jl0 = (warp & 1) * 16 + (lane & 7), il0 = (warp >> 1) * 8 + (lane >> 3);
+  const int jl0 = (warp & 1) * 16 + pr_lane_j(lane), il0 = (warp >> 1) * 8 + pr_lane_i(lane);
 
   // (type, l) rows of consecutive types are consecutive in rowJ / rowI:
   // the chunk's rows are k = 0 .. ntc ltop - 1 from row t0 ltop, and with
@@ -442,7 +441,7 @@ __global__ void __launch_bounds__(FRC_THREADS) k_force_bins(DevProb P, const int
   const int2 t = tiles[blockIdx.x];
   const int i0 = t.x * SPH_T, j0 = t.y * SPH_T;
   const int nv = P.nv;
-  const int jl0 = (warp & 1) * 16 + (lane & 7), il0 = (warp >> 1) * 8 + (lane >> 3);
+  const int jl0 = (warp & 1) * 16 + pr_lane_j(lane), il0 = (warp >> 1) * 8 + pr_lane_i(lane);
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int J = j0 + jl0 + 8 * (q >> 1), I = i0 + il0 + 4 * (q & 1);

@@ -244,6 +244,14 @@ __global__ void k_pair_rows(DevProb P, const SphCoef* __restrict__ coef, double2
   rowI[2 * o + 1] = cmk(c.vif * (c.mAA * a + c.mAB * b), c.vif * (c.mBA * a + c.mBB * b));
 }
 
+// Rows of a lane in the pair kernels: J row (0..7) and I row (0..3).  A 128-bit
+// shared load takes two cycles where lanes i and i ^ 1 (I rows) or i and i ^ 2
+// (J rows) of each half warp read one address, and four otherwise.  With J =
+// lane & 7, I = lane >> 3 the J loads took four: 2.5 per load on the mean against
+// 1.9 now, k_spherical 3.48 -> 3.37 ms and k_force_sph 3.90 -> 3.77 (40 atoms, nv 4600).
+__device__ __forceinline__ int pr_lane_j(int lane) { return (lane & 1) | ((lane >> 1) & 6); }
+__device__ __forceinline__ int pr_lane_i(int lane) { return ((lane >> 1) & 1) | ((lane >> 3) & 2); }
+
 #define PR_MAXA 16  // equivalent atoms per staged chunk (a type with more reads its phases from global)
 #define PR_LT 11    // l count of the specialised kernel (lmax = 10)
 
@@ -282,10 +290,10 @@ __host__ __device__ constexpr int sph_smem_bytes(int lt) {
 
 // One block per 32 x 32 pair tile, 256 threads, bound by the FP64 pipe's
 // issue.  Thread (warp, lane) owns the 2 x 2 pairs J = j0 + jl0 + {0, 8},
-// I = i0 + il0 + {0, 4} with jl0 = 16 (warp & 1) + (lane & 7), il0 =
-// 8 (warp >> 1) + (lane >> 3): a warp reads 8 distinct J rows and 4 distinct
-// I rows per l, 6 shared loads for 24 FP64 operations, each about one cycle
-// (8 or fewer distinct words).  The chunk of types after the current one is
+// I = i0 + il0 + {0, 4} with jl0 = 16 (warp & 1) + pr_lane_j, il0 =
+// 8 (warp >> 1) + pr_lane_i: a warp reads 8 distinct J rows and 4 distinct
+// I rows per l, 6 shared loads of two cycles for 24 FP64 operations.  (2 x 1
+// pairs in 16 warps: 4 loads for 12, 4.5% slower; 12 warps of 2 x 2: spills.)  The chunk of types after the current one is
 // copied by cp.async meanwhile (one block barrier per chunk), and for
 // one-atom types the phase products of a type are formed beside the l sums
 // of the next.  LT: l values (unrolled); GUARD: ltop may be below LT.
@@ -303,7 +311,7 @@ __global__ void __launch_bounds__(SPH_THREADS, 1)
   const int2 t = tiles[blockIdx.x];
   const int i0 = t.x * SPH_T, j0 = t.y * SPH_T;
   const int nv = P.nv, ltop = P.ltop, nat = P.nat, nvpad = P.nvpad;
-  const int jl0 = (warp & 1) * 16 + (lane & 7), il0 = (warp >> 1) * 8 + (lane >> 3);
+  const int jl0 = (warp & 1) * 16 + pr_lane_j(lane), il0 = (warp >> 1) * 8 + pr_lane_i(lane);
 
   // (type, l) rows of consecutive types are consecutive in rowJ / rowI
   auto stage = [&](int st, int t0, const PairChunk& ch) {
