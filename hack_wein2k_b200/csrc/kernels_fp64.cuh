@@ -844,12 +844,14 @@ __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int n
 
 // LO rows: A2 += TUU21 conj(CLM), B2 += TUD21 conj(CLM),
 // C2 = TUU12 conj(ALM) + TDU12 conj(BLM) + TUU22 conj(CLM)  (hns.F:391-433).
-// Block (32 la, 8) over 32 LO rows of an atom: a warp takes 4 of them in turn,
-// lane la.  A row has ALM, BLM, CLM on the atoms of its own type only, and
+// Block (32 la, 8) over 8 LO rows of an atom: a warp takes one of them, lane la.
+// Bound by latency (the copy of the rows, then T per non-zero b, then L):
+// with 32 rows per block, four in turn per warp, 27 us at six atoms, 12.7 now;
+// 62 and 70 us at 100 atoms, where it runs beside the spherical stage.  A row has ALM, BLM, CLM on the atoms of its own type only, and
 // there only at its own l: the sums run over the non-zero b (bits of a ballot;
 // NaN counts as non-zero), 1 + 3 + 5 of 25 for s, p and d rows, and a row
 // that is zero on the atom writes C2 = 0 and leaves L as it is.
-#define LOOPS_ROWS 32
+#define LOOPS_ROWS 8
 __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __restrict__ tns,
                                                     double2* __restrict__ Lop, const double2* __restrict__ Rop,
                                                     const double2* __restrict__ Clo, double2* __restrict__ C2lo) {
@@ -860,7 +862,7 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
   const int nsl2 = (P.lnsmax + 1) * (P.lnsmax + 1);
   const size_t npad = P.npad;
   for (int q = threadIdx.y * 32 + threadIdx.x; q < LOOPS_ROWS * 3 * nsl2; q += 256) {
-    const int r = q / (3 * nsl2), w = (q / nsl2) % 3, b = q % nsl2;
+    const int r = q % LOOPS_ROWS, w = q / LOOPS_ROWS / nsl2, b = q / LOOPS_ROWS % nsl2;
     const int cc = c0 + r;
     double2 v = cmk(0.0, 0.0);
     if (cc < P.nlo) {
@@ -874,15 +876,14 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
   }
   __syncthreads();
   const double2* T = tns + (size_t)P.atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2 + min(la, nsl2 - 1) * L1G_NSL2;
-  for (int u = 0; u < LOOPS_ROWS / 8; u++) {
-    const int r = cy + 8 * u, c = c0 + r;  // warp-uniform
-    if (c >= P.nlo) break;
+  const int r = cy, c = c0 + r;  // warp-uniform
+  if (c < P.nlo) {
     bool nz = false;
     if (la < nsl2)
 #pragma unroll
       for (int w = 0; w < 3; w++) nz |= sX[r][w][la].x != 0.0 || sX[r][w][la].y != 0.0;
     unsigned bits = __ballot_sync(0xffffffffu, nz);
-    if (la >= nsl2) continue;
+    if (la >= nsl2) return;
     double2 da = cmk(0, 0), db = da, dc = da;
     const bool some = bits != 0;
     for (; bits; bits &= bits - 1) {
