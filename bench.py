@@ -21,7 +21,7 @@ of the same crystal (k-point sharding, no collective on the data path).
 `value` is ms per k-point of setup + forces for the whole job (device
 time of K steps, CUDA events on the library's stream, max over ranks, over
 16 N k-points per step).  `fp64_path` times the plain FP64 GPU path (FP64
-spherical kernel, FP64 HNS with library ZGEMM panels, FP64 density
+spherical kernel, FP64 HNS on DMMA, FP64 density
 matrices, every adjoint pair on the FP64 pair kernel) on the same k-points
 and eigenvectors, against the split arm (int8 slice products on tcgen05,
 the adjoint's cross-block spherical pairs as int8 projections); `setup` and `forces` split
@@ -331,11 +331,11 @@ def force_sph_flops(p, block=None):
 
 
 def force_proj_ops(p, nb, S):
-    """int8 ops of the adjoint's spherical projections: output K x 4 nb
-    complex (K = 2 NDF ltop^2 real-harmonic rows), inner NV complex, 8 real
-    ops per complex multiply-add, S(S+1)/2 slice products"""
-    K = 2.0 * p.ndf * p.ltop ** 2
-    return 8.0 * K * 4.0 * nb * p.nv * (S * (S + 1) / 2.0)
+    """int8 ops of the adjoint's spherical projections: per atom 8 ltop^2
+    real rows (2 radial factors x 4 weights per harmonic) x 2 nb real columns,
+    inner NV real, 2 ops per multiply-add, S(S+1)/2 slice products"""
+    rows = 8.0 * p.ndf * p.ltop ** 2
+    return 2.0 * rows * 2.0 * nb * p.nv * (S * (S + 1) / 2.0)
 
 
 def sph_tc_ops(p, S):
@@ -649,7 +649,7 @@ def c4_step_line(args):
     }
 
     if fproj_on:
-        kern["k_split_gemm (adjoint spherical projections, tcgen05 int8, with their operand slicing)"] = (
+        kern["k_fsp_gemm (adjoint spherical projections, tcgen05 int8, with their operand slicing)"] = (
             "tensor", force_proj_ops(p0, NBANDS, fproj_s), ms_fproj_split, "TOP/s", int8_peak)
 
     def rate(w, t, unit):

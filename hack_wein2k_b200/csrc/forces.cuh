@@ -425,9 +425,12 @@ __device__ __forceinline__ int frc_lof(int lm) {
 
 // the default (lapw1gpu_set_force_projection slices -1): 6 slices (at 5 the
 // c1 adjoint's error grew from 2.5e-8 to 1.2e-5 of its largest component),
-// on when the PW rows span 6 blocks (at c1, 4.5 blocks of 1024 rows, the
-// projections took 6.97 ms against 6.09 for the pair kernel alone; at c4,
-// 11.6 blocks, 57.3 against 73.7 ms for the whole adjoint)
+// on when the PW rows span 6 blocks of 1024.  Adjoint in all, pair kernel alone
+// against projections: 1.7 to 3.7 blocks (nv 1706..3790) 1.07-4.21 against
+// 1.36-4.06 ms; 4.5 blocks (the 40-atom supercell) 5.97 against 5.26, but its
+// error grows from 5.4e-12 to 3.9e-10, with any slice count (one pair within
+// 1e-7 of parallel takes hamilt.F's UTOP form there); 11.5 blocks (100 atoms) k_force_sph on every pair alone takes 61
+// ms, where the whole adjoint takes 46.
 #define L1G_FSP_SLICES 6
 #define L1G_FSP_MIN_BLOCKS 6
 

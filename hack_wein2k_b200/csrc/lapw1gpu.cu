@@ -8,7 +8,7 @@
 //   HNS     -> k_hns_alm, k_hns_tmul, k_hns_lo_ops (operands), then
 //              k_tri_gemm (FP64, DMMA) or the split-precision tcgen05 path,
 //              each with its LO-LO block
-//   HORB    -> k_horb_rows, k_horb_pairs per U-atom and l
+//   HORB    -> k_horb_rows (every U-atom and l), k_tri_gemm
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
@@ -516,7 +516,7 @@ int lapw1gpu_forces_stats(lapw1gpu_context* c, lapw1gpu_stats* st) {
   st->ms_spherical = c->fms[1] + c->fms[2];
   st->ms_sph_main = c->fms[2] - c->fms[5];  // k_force_sph
   st->ms_sph_slice = c->fms[6];               // the products of the spherical projections
-  st->ms_table = c->fms[5] - c->fms[6];       // and their other kernels (operand, prefix, bins)
+  st->ms_table = c->fms[5] - c->fms[6];       // and their other kernels (harmonics, exponents, bins)
   st->ms_lo = c->fms[3];        // the step-function sums and the LO columns
   st->ms_hns = c->fms[4];       // the HNS part
   st->ms_total = c->fms[0] + c->fms[1] + c->fms[2] + c->fms[3] + c->fms[4];
@@ -2207,8 +2207,9 @@ static int forces_check(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double* d
 }
 
 // Band-energy gradient (forces.cuh): rho = C f C^H and rhoE = C f eps C^H by
-// library ZGEMM, the PW x PW and LO parts by k_force_sph / k_force_lo, the
-// HNS part through its factors (four ZGEMMs and a per-atom reduction).
+// k_tri_gemm or slice products, the PW x PW and LO parts by k_force_sph /
+// k_force_lo (and the projections of fsp_tc.cuh), the HNS part through its
+// factors (four products and a per-atom reduction).
 int lapw1gpu_forces(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double* d_c, int ldc, int nb, const double* d_occ,
                     const double* d_eps, double* d_grad) {
   int rc = forces_check(c, k, d_c, ldc, nb, d_occ, d_eps, d_grad);

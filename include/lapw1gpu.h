@@ -154,8 +154,8 @@ typedef struct lapw1gpu_stats {
   double kernel_launches;  /* kernels this library launched in the run */
   double ms_sph_main;   /* the spherical contraction kernel alone (k_spherical
                            or k_sph_tc), inside ms_spherical               */
-  double ms_hns_main;   /* the HNS update alone (k_hns_gemm + ZGEMM panels, or
-                           the tcgen05 slice products), inside ms_hns      */
+  double ms_hns_main;   /* the HNS update alone (k_tri_gemm or the tcgen05
+                           slice products), inside ms_hns                  */
   double ms_k_albl;     /* K-a: the matching-coefficient kernel k_albl alone  */
   double ms_table;      /* K-c: the Theta/WARP table kernel k_table alone     */
   double ms_sph_slice;  /* K-a, split path: the two spherical operand slicers
@@ -189,7 +189,7 @@ int lapw1gpu_set_force_slices(lapw1gpu_context* ctx, int slices_density,
  * slices = 0 keeps the FP64 pair kernel for every PW x PW pair; 4..8 forms
  * the pairs of two different blocks of block_rows PW rows (a multiple of
  * 32, at least 64) from int8 slice products of the rows' real-harmonic
- * expansion (addition theorem) with (G c)^T, block by block against the
+ * expansion (addition theorem) with the eigenvectors, block by block against the
  * running sum of the blocks before; the pairs inside a block stay on the
  * FP64 pair kernel.  slices = -1 (the default, with 1024-row blocks): 6
  * slices when the PW rows span at least 6 blocks, else the pair kernel. */
@@ -346,14 +346,16 @@ int lapw1gpu_setup_batch(lapw1gpu_context* ctx, lapw1gpu_kpoint* const* kps,
 /* Tunables of the context (tile and schedule parameters) and the
  * autotuner that picks them by timing candidates on a k-point. */
 typedef struct {
-  int hns_diag_b;   /* FP64 HNS: diagonal block of the blocked update (256..2048) */
+  int hns_diag_b;   /* accepted as before (a multiple of 64), without effect:
+                       the FP64 HNS update is one product without blocks     */
   int split_group;  /* split HNS: row tiles per L2 rasterisation group           */
   int sph_tc;       /* split: spherical part on tcgen05 (1) or FP64 (0)          */
-  int batch_sets;   /* concurrent k-point chains in a batch (1..4)               */
+  int batch_sets;   /* concurrent k-point chains in a batch (1..4); until it is
+                       set, 4 for batches of N up to 1088 and else the default */
   int sph_kblock;   /* split: K bytes per k_sph_tc pipeline stage, 64 (four-deep
                        ring of 64-byte swizzled rows) or 128 (two stages of
-                       128-byte rows; up to 5 slices, else 64 is used;
-                       the default)                                           */
+                       128-byte rows; up to 5 slices, else 64 is used).
+                       Until it is set, 128 unless 64 pads K less           */
   double ms_best;   /* setup time of the tuned k-point with the choices, ms      */
 } lapw1gpu_tuning;
 int lapw1gpu_get_tuning(lapw1gpu_context* ctx, lapw1gpu_tuning* t);
