@@ -86,7 +86,7 @@ struct lapw1gpu_context {
   bool fproj_last = false;  // the last forces call formed spherical projections
   std::vector<cudaEvent_t> fpev;  // timed forces call: around each chunk of the projections
   int fpev_used = 0;
-  // per scratch set: the stream that prepares the split HNS operands while
+  // per scratch set: the stream that prepares the HNS operands while
   // the spherical stage runs, and its fork/join events
   cudaStream_t aux[L1G_MAX_SETS] = {};
   cudaEvent_t auxf[L1G_MAX_SETS] = {}, auxj[L1G_MAX_SETS] = {};
@@ -1095,12 +1095,13 @@ static double alg_flops(const lapw1gpu_kpoint* k) {
 // The stage sequence of one k-point on stream s with scratch set `set`.
 // ev: events to record between stages (null where nobody asks for timings: a
 // record per kernel costs the host and the stream about 2 us each).
-// hamilt_done: recorded after HAMILT.  Host-side work
+// hamilt_done: recorded after HAMILT.  chained: one of several concurrent
+// k-points of a batch.  Host-side work
 // is limited to launches: every buffer and tile list already exists when
 // the same k-point ran once before, so the sequence can be captured.
 static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, double2* d_hs, int ldhs,
                            double2* d_hsdiag, cudaStream_t s, int set, const cudaEvent_t* ev, int* nlaunch,
-                           HnsPipe* hp = nullptr, cudaEvent_t hamilt_done = nullptr) {
+                           HnsPipe* hp = nullptr, cudaEvent_t hamilt_done = nullptr, bool chained = false) {
   DevProb P = k->P;
   const int n = k->n, nv = k->nv, ltop = k->ltop, ndf = k->ndf, nat = k->nat;
   P.al = (double*)c->sbuf(set, "al", sizeof(double) * (size_t)nat * ltop * k->nvpad);
@@ -1124,12 +1125,17 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
   CK(cudaGetLastError());
   if (ev) CK(cudaEventRecord(ev[1], s));
 
-  // HNS operand buffers; in split precision the operands (ALM/BLM/CLM, L,
-  // the LO terms, row exponents and int8 slices) are prepared on the set's
+  // HNS operand buffers; the operands (ALM/BLM/CLM, L, the LO terms; in split
+  // precision also row exponents and int8 slices) are prepared on the set's
   // auxiliary stream while the spherical stage runs on s: they read AL/BL
-  // and the phases only.  s joins it before the HNS products.
+  // and the phases only.  s joins it before the HNS products.  FP64, against one
+  // stream: one atom 0.176 -> 0.163 ms, six 0.464 -> 0.436, 40 atoms 10.17 ->
+  // 10.06.  The chains of an FP64 batch overlap one another instead: forks
+  // gave 16 k-points of six atoms 6%, and its first pass, which captures
+  // twice the streams, took 4.0 ms instead of 3.25.
   const bool hns = (stages & 2) && !k->nohns;
-  const bool hns_fork = hns && c->prec == LAPW1GPU_PREC_SPLIT;
+  const bool hns_split = hns && c->prec == LAPW1GPU_PREC_SPLIT;
+  const bool hns_fork = hns_split || (hns && !chained);
   const int nsl2 = (k->lnsmax + 1) * (k->lnsmax + 1);
   const int Khns = ndf * 2 * nsl2;
   double2 *Lop = nullptr, *Rop = nullptr, *Clo = nullptr, *C2lo = nullptr;
@@ -1142,16 +1148,16 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     if (!Lop || !Rop || !Clo || !C2lo) return LAPW1GPU_ERR_NOMEM;
   }
   if (hns_fork) {
-    // on the set's auxiliary stream: the operands, their int8 slices and
-    // the LO-LO block T = C2 CLM^T (tensor cores, added after the HNS products)
+    // on the set's auxiliary stream: the operands and, split, their int8 slices
+    // and the LO-LO block T = C2 CLM^T (tensor cores, added after the HNS products)
     cudaStream_t a = c->aux[set];
     CK(cudaEventRecord(c->auxf[set], s));
     CK(cudaStreamWaitEvent(a, c->auxf[set], 0));
     int rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, a, &nl);
-    if (!rc)
+    if (!rc && hns_split)
       rc = split_hns_gemm(c, k, set, n, k->npad, Khns, Lop, Rop, d_hs, ldhs, c->slices_hns, a, &nl, nullptr,
                           nullptr, 0, 1);
-    if (!rc && k->nlo > 0) {
+    if (!rc && hns_split && k->nlo > 0) {
       double2* T = (double2*)c->sbuf(set, "hnsLoT", sizeof(double2) * (size_t)k->nlo * k->nlo);
       if (!T) return LAPW1GPU_ERR_NOMEM;
       rc = split_rect_gemm(c, k, set, k->nlo, k->nlo, ndf * nsl2, C2lo, k->nlo, Clo, k->nlo, T, k->nlo,
@@ -1246,13 +1252,15 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     // ---- K-ns ----
     const int K = Khns;
     int rc = LAPW1GPU_OK;
-    if (hns_fork) {
+    if (hns_fork)
       CK(cudaStreamWaitEvent(s, c->auxj[set], 0));
+    else
+      rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, s, &nl);
+    if (rc) return rc;
+    if (hns_split) {
       rc = split_hns_gemm(c, k, set, n, k->npad, K, Lop, Rop, d_hs, ldhs, c->slices_hns, s, &nl, hp,
                           ev ? ev + 14 : nullptr, 0, 2);
     } else {
-      rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, s, &nl);
-      if (rc) return rc;
       if (ev) CK(cudaEventRecord(ev[14], s));
       // column group by column group (groups whose columns reach the LO block
       // are recorded after it)
@@ -1271,7 +1279,7 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     if (k->nlo > 0) {
       // C2 CLM^T on the LO block: FP64 added in place; in split precision
       // the auxiliary stream's tensor-core product, its lower triangle into HS
-      if (hns_fork) {
+      if (hns_split) {
         double2* T = (double2*)c->sbuf(set, "hnsLoT", sizeof(double2) * (size_t)k->nlo * k->nlo);
         if (!T) return LAPW1GPU_ERR_NOMEM;
         nl++;
@@ -1396,7 +1404,7 @@ static int batch_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int n
     const int set = i % sets;
     cudaStream_t s = set ? c->side[set] : c->stream;
     int rc = kpoint_run_impl(c, kps[i], stages, reinterpret_cast<double2*>(d_hs[i]), ldhs[i],
-                             reinterpret_cast<double2*>(d_hsdiag[i]), s, set, nullptr, nl);
+                             reinterpret_cast<double2*>(d_hsdiag[i]), s, set, nullptr, nl, nullptr, nullptr, sets > 1);
     if (rc) return rc;
   }
   for (int q = 1; q < sets; q++) {
