@@ -301,7 +301,7 @@ template <int LT, bool GUARD>
 __global__ void __launch_bounds__(SPH_THREADS, 1)
     k_spherical(DevProb P, const int2* __restrict__ tiles, const double2* __restrict__ rowJ,
                 const double2* __restrict__ rowI, const double2* __restrict__ tab, TabDesc T, double2* __restrict__ hs,
-                int ld, double2* __restrict__ hsdiag) {
+                int ld, double2* __restrict__ hsdiag, int* __restrict__ status) {
   constexpr int TC = pr_tc(LT);
   extern __shared__ double2 sm2[];
   double2* sJ = sm2;                       // [2][TC][LT][SPH_T]
@@ -488,8 +488,10 @@ __global__ void __launch_bounds__(SPH_THREADS, 1)
     ch = nx;
     st ^= 1;
   }
-  // interstitial + write (hamilt.F:289-345, 459-466, calkpt.F:164)
+  // interstitial + write (hamilt.F:289-345, 459-466, calkpt.F:164); a non-finite
+  // written element sets L1G_STATUS_NONFINITE
   const int nx = 2 * T.d1 + 1, ny = 2 * T.d2 + 1;
+  bool bad = false;
 #pragma unroll
   for (int v = 0; v < 2; v++) {
     const int I = i0 + il0 + 4 * v;
@@ -514,8 +516,10 @@ __global__ void __launch_bounds__(SPH_THREADS, 1)
         hs[(size_t)I * ld + J] = s;  // S upper: HS(J,I)
         hs[(size_t)J * ld + I] = h;  // H lower: HS(I,J)
       }
+      bad |= l1g_nonfinite(s) | l1g_nonfinite(h);
     }
   }
+  if (bad) atomicOr(status, L1G_STATUS_NONFINITE);
 }
 
 // ---------------------------------------------------------------------
@@ -612,8 +616,7 @@ __device__ __forceinline__ double2 lo_dot(const DevProb& P, int nm, const double
 }
 
 // cols[groups[y]]: the group's first column (mo1 = -l).  status: when non-null,
-// a non-finite written element sets L1G_STATUS_NONFINITE (the split path's
-// writers check what they write).
+// a non-finite written element sets L1G_STATUS_NONFINITE.
 __global__ void __launch_bounds__(128) k_lo(DevProb P, const LoCol* __restrict__ cols, const int* __restrict__ groups,
                                             double2* __restrict__ hs, int ld, double2* __restrict__ hsdiag,
                                             int* __restrict__ status) {

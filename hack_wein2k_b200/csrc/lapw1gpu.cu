@@ -1167,7 +1167,6 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     CK(cudaEventRecord(c->auxj[set], a));
   }
 
-  bool sph_tc_used = false;  // the spherical stage ran on the tensor-core kernel
   if (stages & 1) {
     // ---- K-c table + K-b spherical ----
     size_t ntab = (size_t)(2 * k->tab.d1 + 1) * (2 * k->tab.d2 + 1) * (2 * k->tab.d3 + 1);
@@ -1187,7 +1186,6 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     if (c->prec == LAPW1GPU_PREC_SPLIT && c->sph_tc && sph_tc_supported(c->slices)) {
       int rc = sph_tc_dispatch(c, k, set, P, coef, tab, d_hs, ldhs, d_hsdiag, s, &nl, ev ? ev + 12 : nullptr, sp);
       if (rc) return rc;
-      sph_tc_used = true;
     } else {
       int ntiles = 0;
       const int2* tl = tiles_tri(k, "sph", nv, SPH_T, &ntiles);
@@ -1214,10 +1212,10 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
           nl++;
           if (lt11)
             k_spherical<PR_LT, false><<<(unsigned)(t1 - t0), SPH_THREADS, smem, s>>>(P, tl + t0, rowJ, rowI, tab, k->tab,
-                                                                                     d_hs, ldhs, d_hsdiag);
+                                                                                     d_hs, ldhs, d_hsdiag, c->d_status);
           else
             k_spherical<SPH_LMAX, true><<<(unsigned)(t1 - t0), SPH_THREADS, smem, s>>>(P, tl + t0, rowJ, rowI, tab,
-                                                                                       k->tab, d_hs, ldhs, d_hsdiag);
+                                                                                       k->tab, d_hs, ldhs, d_hsdiag, c->d_status);
         }
         if (sp && sp->col[g + 1] <= nv) {
           CK(cudaEventRecord(sp->sev[g], s));
@@ -1267,7 +1265,7 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
       const int G = hp && hp->groups > 0 ? hp->groups : 1;
       for (int g = 0; g < G && !rc; g++) {
         rc = launch_tri(c, n, G > 1 ? hp->col[g] : 0, G > 1 ? hp->col[g + 1] : n, K, Lop, k->npad, Rop, k->npad, d_hs,
-                        ldhs, 0, nullptr, s, &nl);
+                        ldhs, 0, c->d_status, s, &nl);
         if (G > 1 && !rc && hp->col[g + 1] <= nv) {
           CK(cudaEventRecord(hp->ev[g], s));
           hp->recorded[g] = true;
@@ -1285,7 +1283,7 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
         nl++;
         k_add_lower<<<dim3((k->nlo + 127) / 128, k->nlo), 128, 0, s>>>(nv, k->nlo, T, d_hs, ldhs, c->d_status);
       } else if (int rc2 = launch_tri(c, k->nlo, 0, k->nlo, ndf * nsl2, C2lo, k->nlo, Clo, k->nlo,
-                                      d_hs + (size_t)nv * ldhs + nv, ldhs, 0, nullptr, s, &nl)) {
+                                      d_hs + (size_t)nv * ldhs + nv, ldhs, 0, c->d_status, s, &nl)) {
         return rc2;
       }
     }
@@ -1311,11 +1309,10 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     CK(cudaGetLastError());
   }
   if (ev) CK(cudaEventRecord(ev[5], s));
-  // Non-finite elements: the split path's writers (k_sph_tc, k_lo, the
-  // split HNS epilogue, k_add_lower) and HORB's product check what they
-  // write; the scan of HS and HSDIAG is needed when the spherical stage did
-  // not run (HS came from the caller) or ran on the FP64 kernel.
-  const bool checked = sph_tc_used;
+  // Non-finite elements: every writer of HS and HSDIAG checks what it writes
+  // (40 atoms: the scan took 74 us).  The scan is needed when the spherical
+  // stage did not run: HS came from the caller.
+  const bool checked = (stages & 1) != 0;
   if (!checked) {
     nl++;
     k_check_finite<<<1184, 256, 0, s>>>(n, d_hs, ldhs, d_hsdiag, c->d_status);
