@@ -112,3 +112,20 @@ def test_projection_tiles(ctx, slices, nb, block, lmax):
         ctx.set_force_slices(6, 6)
         ctx.set_force_projection(-1, 1024)
     assert np.abs(out[1] - out[0]).max() <= (64 * (slices + 1) * 2.0 ** (-7 * slices) + 1e-9) * np.abs(out[0]).max()
+
+
+# one writer of HS each: k_spherical, k_lo, the HNS product
+@pytest.mark.parametrize("field,lo,stages", [("e", (), 1), ("alo", (0, 1), 1), ("tns", (), 3)])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_fp64_writers_report_nonfinite(ctx, field, lo, stages, value):
+    ctx.set_precision(lapw1gpu.PREC_FP64)
+    p = _plain(5.0, lo_l=lo)
+    a = np.array(getattr(p, field), copy=True)
+    if field == "alo":  # every local orbital's coefficient
+        a[...] = value
+    else:
+        a.flat[0] = value
+    with pytest.raises(lapw1gpu.Lapw1GpuError) as ei:
+        ctx.setup(p.copy(**{field: a}), stages=stages)
+    assert ei.value.code == 4
+    ctx.setup(p, stages=stages)
