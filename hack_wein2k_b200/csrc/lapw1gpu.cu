@@ -124,11 +124,10 @@ struct lapw1gpu_context {
   int hns_diag_b = 512;    // kept for callers that set it; the FP64 HNS update is one product without blocks
   int split_group = 16;    // split HNS: row tiles per rasterisation group
   int sph_tc = 1;          // split precision: spherical part on tcgen05 (1) or FP64 (0)
-  int sph_kb = 128;        // k_sph_tc: bytes of K per pipeline stage (64: deep ring, 128: two stages)
-  int batch_sets = 2;      // concurrent k-point chains in a batch
-  // chosen by the caller or the autotuner; until then a rule on the sizes
-  // decides (sph_kb128, batch_chains)
-  bool sph_kb_set = false, batch_sets_set = false;
+  // chosen by the caller or the autotuner; 0: a rule on the sizes decides
+  // (sph_kb128, batch_chains)
+  int sph_kb = 0;          // k_sph_tc: bytes of K per pipeline stage (64: deep ring, 128: two stages)
+  int batch_sets = 0;      // concurrent k-point chains in a batch
   int test_never_wait = 0; // test hook: the spherical tensor kernel's consumer wait runs out
   int last_launches = 0;   // kernels launched by the last call (a library product counts as one)
   std::map<std::string, DevBuf> bufs;
@@ -1050,7 +1049,7 @@ static bool sph_tc_supported(int S) { return S >= 4 && S <= 7; }
 // halved count of blocks is up to 2.5% faster (K = 256: 1.59 against 1.62).
 static bool sph_kb128(const lapw1gpu_context* c, int Kp) {
   if (c->slices > 5) return false;
-  if (c->sph_kb_set) return c->sph_kb == 128;
+  if (c->sph_kb) return c->sph_kb == 128;
   return (Kp + 63) / 64 * 64 == (Kp + 127) / 128 * 128;
 }
 
@@ -1386,7 +1385,7 @@ int lapw1gpu_kpoint_run(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, dou
 // two (four k-points of N = 4950: kernels that fill the SMs anyway).
 #define L1G_SMALL_N 1088
 static int batch_chains(const lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int nk) {
-  if (c->batch_sets_set) return std::max(1, std::min(c->batch_sets, L1G_MAX_SETS));
+  if (c->batch_sets) return c->batch_sets;
   int n = 0;
   for (int i = 0; i < nk; i++) n = std::max(n, kps[i]->n);
   return n <= L1G_SMALL_N ? L1G_MAX_SETS : 2;
@@ -1420,7 +1419,7 @@ int lapw1gpu_setup_batch(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int n
   std::vector<uintptr_t> key = {(uintptr_t)nk,         (uintptr_t)stages,        (uintptr_t)c->prec,
                                 (uintptr_t)(c->slices * 16 + c->slices_hns), (uintptr_t)c->hns_diag_b,
                                 (uintptr_t)c->split_group,
-                                (uintptr_t)c->sph_tc,  (uintptr_t)(c->sph_kb * 2 + c->sph_kb_set),
+                                (uintptr_t)c->sph_tc,  (uintptr_t)c->sph_kb,
                                 (uintptr_t)batch_chains(c, kps, nk),
                                 (uintptr_t)c->test_never_wait};
   for (int i = 0; i < nk; i++) {
@@ -1503,17 +1502,15 @@ int lapw1gpu_get_tuning(lapw1gpu_context* c, lapw1gpu_tuning* t) {
 
 int lapw1gpu_set_tuning(lapw1gpu_context* c, const lapw1gpu_tuning* t) {
   if (!c || !t) return LAPW1GPU_ERR_ARG;
-  if (t->hns_diag_b < TRI_COLS || t->hns_diag_b % TRI_COLS || t->split_group < 1 || t->batch_sets < 1 ||
+  if (t->hns_diag_b < TRI_COLS || t->hns_diag_b % TRI_COLS || t->split_group < 1 || t->batch_sets < 0 ||
       t->batch_sets > L1G_MAX_SETS || (t->sph_tc != 0 && t->sph_tc != 1) ||
-      (t->sph_kblock != 64 && t->sph_kblock != 128))
+      (t->sph_kblock != 0 && t->sph_kblock != 64 && t->sph_kblock != 128))
     return LAPW1GPU_ERR_RANGE;
   c->hns_diag_b = t->hns_diag_b;
   c->split_group = t->split_group;
   c->sph_tc = t->sph_tc;
-  // (a value that is reported already is not a choice: callers that change
+  // (0, reported until a value is chosen, keeps the rule: callers that change
   // one field write the others back)
-  if (t->batch_sets != c->batch_sets) c->batch_sets_set = true;
-  if (t->sph_kblock != c->sph_kb) c->sph_kb_set = true;
   c->batch_sets = t->batch_sets;
   c->sph_kb = t->sph_kblock;
   return LAPW1GPU_OK;
@@ -1563,9 +1560,10 @@ int lapw1gpu_autotune(lapw1gpu_context* c, lapw1gpu_kpoint* kp, double* d_hs, in
     // the K block (and with it the ring depth) of k_sph_tc: 128-byte blocks
     // exist up to 5 slices
     if (!rc && c->sph_tc && c->slices <= 5) {
-      if (!c->sph_kb_set) c->sph_kb = sph_kb128(c, 2 * round_up(2 * kp->ndf, 16)) ? 128 : 64;  // the value held
-      c->sph_kb_set = true;
+      const int chosen = c->sph_kb;
+      c->sph_kb = sph_kb128(c, 2 * round_up(2 * kp->ndf, 16)) ? 128 : 64;  // the value held
       rc = tune(&c->sph_kb, {64, 128}, T_SPH);
+      if (rc) c->sph_kb = chosen;
     }
     if (!rc) rc = tune(&c->split_group, {4, 8, 16, 32}, T_HNS);
   }
@@ -1580,6 +1578,9 @@ int lapw1gpu_autotune(lapw1gpu_context* c, lapw1gpu_kpoint* kp, double* d_hs, in
   if (rc) return rc;
   if (out) {
     lapw1gpu_get_tuning(c, out);
+    // where the rules decide, what they give for this k-point
+    if (!out->batch_sets) out->batch_sets = batch_chains(c, &kp, 1);
+    if (!out->sph_kblock) out->sph_kblock = sph_kb128(c, 2 * round_up(2 * kp->ndf, 16)) ? 128 : 64;
     out->ms_best = total_best;
   }
   return LAPW1GPU_OK;

@@ -350,14 +350,17 @@ typedef struct {
                        the FP64 HNS update is one product without blocks     */
   int split_group;  /* split HNS: row tiles per L2 rasterisation group           */
   int sph_tc;       /* split: spherical part on tcgen05 (1) or FP64 (0)          */
-  int batch_sets;   /* concurrent k-point chains in a batch (1..4); until it is
-                       set, 4 for batches of N up to 1088 and else the default */
+  int batch_sets;   /* concurrent k-point chains in a batch (1..4), or 0 (the
+                       default): 4 for batches of N up to 1088, else 2        */
   int sph_kblock;   /* split: K bytes per k_sph_tc pipeline stage, 64 (four-deep
                        ring of 64-byte swizzled rows) or 128 (two stages of
-                       128-byte rows; up to 5 slices, else 64 is used).
-                       Until it is set, 128 unless 64 pads K less           */
+                       128-byte rows; up to 5 slices, else 64 is used), or 0
+                       (the default): 128 unless 64 pads K less             */
   double ms_best;   /* setup time of the tuned k-point with the choices, ms      */
 } lapw1gpu_tuning;
+/* get_tuning reports 0 in batch_sets and sph_kblock while the rules above
+ * decide; any other value that set_tuning is given is a choice and is what
+ * runs.  lapw1gpu_autotune's out holds what runs for its k-point. */
 int lapw1gpu_get_tuning(lapw1gpu_context* ctx, lapw1gpu_tuning* t);
 int lapw1gpu_set_tuning(lapw1gpu_context* ctx, const lapw1gpu_tuning* t);
 /* Time the candidates of every tunable of the current precision on kp

@@ -70,6 +70,57 @@ def test_batch_equals_single_runs(ctx, prec, slices, sets):
 
 
 @pytest.mark.gpu
+def test_chosen_chains_are_the_chains_that_run(ctx):
+    """batch_sets on a context that nothing was set on: 0 (by rule) takes four
+    chains for k-points of N <= 1088, every other value is what runs, its
+    former default of 2 included.  A chain shows as its scratch set on the
+    device; results are single runs' whatever the chains."""
+    dev = torch.device("cuda", ctx.device)
+    ctx.set_precision(lapw1gpu.PREC_FP64)
+    probs = [synth.small_case("lo", rkmax=10.0)] * 4
+    p = probs[0]
+    assert p.n <= 1088
+    ref = _single(ctx, probs[:1], dev)[0]
+    operand = 16 * p.ndf * 2 * (p.lnsmax + 1) ** 2 * p.n  # HNS L or R of one chain, bytes
+
+    def used(sets):
+        with lapw1gpu.Context(ctx.device) as c:
+            assert c.tuning()["batch_sets"] == 0 and c.tuning()["sph_kblock"] == 0
+            if sets:
+                c.set_tuning(batch_sets=sets)
+            assert c.tuning()["batch_sets"] == sets
+            kps = [c.upload(q) for q in probs]
+            hs, hd = _alloc(probs, dev)
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info(dev)[0]
+            c.setup_batch(kps, [h.data_ptr() for h in hs], [q.n for q in probs], [d.data_ptr() for d in hd])
+            free -= torch.cuda.mem_get_info(dev)[0]
+            for h, d in zip(hs, hd):
+                assert np.array_equal(_host(h), ref[0]) and np.array_equal(d.cpu().numpy(), ref[1])
+            for k in kps:
+                k.free()
+        return free
+
+    used(0)  # what a first context allocates once is not counted
+    mem = {sets: used(sets) for sets in (0, 1, 2, 4)}
+    assert mem[0] - mem[2] >= 4 * operand and mem[4] - mem[2] >= 4 * operand, mem
+    assert mem[2] - mem[1] >= 2 * operand, mem
+
+
+@pytest.mark.gpu
+def test_choice_of_the_k_block_is_kept(ctx):
+    with lapw1gpu.Context(ctx.device) as c:
+        for kb in (128, 64, 0):
+            c.set_tuning(sph_kblock=kb)
+            c.set_tuning(split_group=8)  # the other fields are written back
+            assert c.tuning()["sph_kblock"] == kb and c.tuning()["batch_sets"] == 0
+        for bad in (dict(batch_sets=-1), dict(batch_sets=5), dict(sph_kblock=32)):
+            with pytest.raises(lapw1gpu.Lapw1GpuError) as e:
+                c.set_tuning(**bad)
+            assert e.value.code == 7  # LAPW1GPU_ERR_RANGE
+
+
+@pytest.mark.gpu
 def test_batch_against_oracle(ctx):
     dev = torch.device("cuda", ctx.device)
     ctx.set_precision(lapw1gpu.PREC_FP64)
