@@ -54,6 +54,7 @@ struct DevBuf {
 
 #define L1G_MAX_SETS 4  // concurrent k-point chains in a batch (scratch sets)
 #define L1G_MAX_GROUPS 16
+#define L1G_FSP_BYTES (16ull << 30)
 #define L1G_STAGE_MAX (256u << 10)  // an upload's arrays up to this size go through page-locked staging
 
 // Column groups of HS: the spherical contraction and the HNS update run
@@ -128,6 +129,9 @@ struct lapw1gpu_context {
   // (sph_kb128, batch_chains)
   int sph_kb = 0;          // k_sph_tc: bytes of K per pipeline stage (64: deep ring, 128: two stages)
   int batch_sets = 0;      // concurrent k-point chains in a batch
+  DevBuf fsp;                          // the spherical projections' int8 operands (fsp_products)
+  size_t fsp_budget = L1G_FSP_BYTES;   // bytes they may take,
+  size_t test_fsp_fit = SIZE_MAX;      // and (test hook) what an allocation of them may take
   int test_never_wait = 0; // test hook: the spherical tensor kernel's consumer wait runs out
   int last_launches = 0;   // kernels launched by the last call (a library product counts as one)
   std::map<std::string, DevBuf> bufs;
@@ -178,13 +182,49 @@ struct lapw1gpu_context {
       }
       b.ptr = nullptr;
       b.bytes = 0;
-      if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-      }
+      if (!dev_malloc(&b.ptr, bytes)) return nullptr;
       b.bytes = bytes;
     }
     return b.ptr;
+  }
+  // cudaMalloc; where it fails, once more without the projections' operands,
+  // which the next adjoint cuts to the memory that it finds
+  bool dev_malloc(void** p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    *p = nullptr;
+    if (!fsp.ptr) return false;
+    fsp_release();
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  void fsp_release() {
+    if (fsp.ptr) {
+      cudaDeviceSynchronize();  // a queued adjoint may still use it (no captured batch does)
+      cudaFree(fsp.ptr);
+    }
+    fsp = DevBuf();
+  }
+  // the projections' operand buffer, or nullptr where so much does not fit
+  // beside the memory in use (what is held then stays as it is)
+  void* fsp_buf(size_t bytes) {
+    if (fsp.bytes >= bytes) return fsp.ptr;
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (std::min(avail + fsp.bytes, test_fsp_fit) < bytes) return nullptr;
+    fsp_release();
+    if (cudaMalloc(&fsp.ptr, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      fsp.ptr = nullptr;
+      return nullptr;
+    }
+    fsp.bytes = bytes;
+    return fsp.ptr;
   }
   // scratch of one set: buffers of concurrent k-point chains never alias
   void* sbuf(int set, const char* name, size_t bytes) {
@@ -247,10 +287,7 @@ static const int2* kp_tiles(lapw1gpu_kpoint* k, const std::string& key, int* cou
   std::vector<int2> t;
   make(t);
   int2* d = nullptr;
-  if (t.empty() || cudaMalloc(&d, sizeof(int2) * t.size()) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
+  if (t.empty() || !k->ctx->dev_malloc((void**)&d, sizeof(int2) * t.size())) return nullptr;
   // The list must be on the device before any stream's kernel reads it: a
   // plain cudaMemcpy of up to 64 KB from pageable memory returns while its
   // copy is still queued on the legacy stream, which the context's
@@ -438,6 +475,7 @@ int lapw1gpu_finalize(lapw1gpu_context* c) {
   for (auto& kv : c->bufs)
     if (kv.second.ptr) cudaFree(kv.second.ptr);
   for (auto& kv : c->tiles) cudaFree(kv.second.first);
+  c->fsp_release();
   if (c->async_pending && c->async_k) lapw1gpu_kpoint_free(c->async_k);
   if (c->h_async_status) cudaFreeHost(c->h_async_status);
   if (c->h_status) cudaFreeHost(c->h_status);
@@ -553,6 +591,15 @@ int lapw1gpu_host_unregister(lapw1gpu_context* c, void* ptr) {
 int lapw1gpu_test_wait_timeout(lapw1gpu_context* c, int on) {
   if (!c || (on != 0 && on != 1)) return LAPW1GPU_ERR_ARG;
   c->test_never_wait = on;
+  return LAPW1GPU_OK;
+}
+
+int lapw1gpu_test_projection_bytes(lapw1gpu_context* c, size_t budget, size_t fit) {
+  if (!c) return LAPW1GPU_ERR_ARG;
+  CK(cudaSetDevice(c->device));
+  c->fsp_release();
+  c->fsp_budget = budget ? budget : L1G_FSP_BYTES;
+  c->test_fsp_fit = fit ? fit : SIZE_MAX;
   return LAPW1GPU_OK;
 }
 
@@ -737,7 +784,7 @@ static int kpoint_upload_impl(lapw1gpu_context* ctx, const lapw1gpu_problem* p, 
       delete k;
       return LAPW1GPU_ERR_NOMEM;
     }
-  } else if (cudaMalloc(&k->arena, off) != cudaSuccess) {
+  } else if (!ctx->dev_malloc(&k->arena, off)) {
     cudaGetLastError();
     delete k;
     return LAPW1GPU_ERR_NOMEM;
@@ -1894,12 +1941,10 @@ int lapw1gpu_setup(lapw1gpu_context* c, const lapw1gpu_problem* p, double* hs, i
 }
 
 // The spherical projections of all atoms (fsp_tc.cuh) on stream s.  The int8
-// operands of as many atoms as L1G_FSP_BYTES holds are built at a time (half
-// of it again and again where that much cannot be allocated).  timed: events
+// operands of as many atoms as the context's budget holds are built at a time
+// (half of it again and again where that much does not fit beside the memory
+// in use).  timed: events
 // around each chunk's operands and products.
-#ifndef L1G_FSP_BYTES
-#define L1G_FSP_BYTES (16ull << 30)
-#endif
 extern "C++" {
 template <int S>
 static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& P, const SphCoef* coef,
@@ -1914,7 +1959,7 @@ static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& 
   std::vector<int> at;
   int8_t *A = nullptr, *B = nullptr;
   int* exA = nullptr;
-  for (size_t budget = L1G_FSP_BYTES;; budget /= 2) {
+  for (size_t budget = c->fsp_budget;;) {
     size_t needA = 0, needB = 0;
     at.assign(1, 0);
     for (int a0 = 0; a0 < ndf;) {
@@ -1925,11 +1970,16 @@ static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& 
       needB = std::max(needB, (size_t)(a1 - a0));
       at.push_back(a0 = a1);
     }
-    A = (int8_t*)c->buf("fspA", needA * typeA);
-    B = A ? (int8_t*)c->buf("fspB", needB * atomB) : nullptr;
-    exA = B ? (int*)c->buf("fspExA", sizeof(int) * needA * MT * 128 * nblk) : nullptr;
-    if (exA) break;
+    // A, B (multiples of 1024 bytes) and the exponents of A
+    const size_t need = needA * typeA + needB * atomB + sizeof(int) * needA * MT * 128 * nblk;
+    A = (int8_t*)c->fsp_buf(need);
+    if (A) {
+      B = A + needA * typeA;
+      exA = (int*)(B + needB * atomB);
+      break;
+    }
     if ((int)at.size() == ndf + 1) return LAPW1GPU_ERR_NOMEM;  // one atom at a time already
+    budget = std::min(budget, need) / 2;
   }
   if (!c->smem((const void*)fsptc::k_fsp_gemm<S>, Cf::SMEM)) return LAPW1GPU_ERR_CUDA;
   for (size_t q = 0; q + 1 < at.size(); q++) {

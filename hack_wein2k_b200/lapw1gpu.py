@@ -35,6 +35,7 @@ EXPORTS = [
     "lapw1gpu_setup_async", "lapw1gpu_setup_wait",
     "lapw1gpu_hns_noalloc", "lapw1gpu_forces", "lapw1gpu_setup_batch", "lapw1gpu_get_tuning",
     "lapw1gpu_set_tuning", "lapw1gpu_autotune", "lapw1gpu_set_slices", "lapw1gpu_test_wait_timeout",
+    "lapw1gpu_test_projection_bytes",
     "lapw1gpu_last_launches", "lapw1gpu_host_register", "lapw1gpu_host_unregister", "lapw1gpu_forces_stats",
     "lapw1gpu_forces_batch", "lapw1gpu_set_force_slices", "lapw1gpu_set_force_projection",
     "lapw1gpu_seclr4",
@@ -100,6 +101,7 @@ def load(path: Optional[str] = None):
     lib.lapw1gpu_set_tuning.argtypes = [vp, C.POINTER(Tuning)]
     lib.lapw1gpu_autotune.argtypes = [vp, vp, C.c_void_p, C.c_int, C.c_void_p, C.POINTER(Tuning)]
     lib.lapw1gpu_test_wait_timeout.argtypes = [vp, C.c_int]
+    lib.lapw1gpu_test_projection_bytes.argtypes = [vp, C.c_size_t, C.c_size_t]
     lib.lapw1gpu_last_launches.argtypes = [vp]
     lib.lapw1gpu_forces_stats.argtypes = [vp, C.POINTER(CStats)]
     lib.lapw1gpu_forces_batch.argtypes = [vp, C.POINTER(vp), C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_int),
@@ -223,6 +225,11 @@ class Context:
         """Test hook (lapw1gpu_test_wait_timeout): make the spherical tensor
         kernel's consumer wait run out on later split-precision runs."""
         _check("lapw1gpu_test_wait_timeout", self.lib.lapw1gpu_test_wait_timeout(self.h, 1 if on else 0))
+
+    def test_projection_bytes(self, budget: int = 0, fit: int = 0) -> None:
+        """Test hook (lapw1gpu_test_projection_bytes): byte budget of the
+        projections' operands and what of it fits on the device."""
+        _check("lapw1gpu_test_projection_bytes", self.lib.lapw1gpu_test_projection_bytes(self.h, budget, fit))
 
     def setup(self, prob: Problem, stages: int = 7, hs: Optional[np.ndarray] = None,
               hsdiag: Optional[np.ndarray] = None, stats: bool = False):

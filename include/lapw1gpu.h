@@ -252,6 +252,14 @@ void* lapw1gpu_stream(lapw1gpu_context* ctx);
  * default) restores normal runs. */
 int lapw1gpu_test_wait_timeout(lapw1gpu_context* ctx, int on);
 
+/* Test hook of the adjoint's spherical projections, whose int8 operands are
+ * built for as many atoms at a time as a byte budget holds.  No counterpart
+ * in the reference.  budget: that budget, 0 for the library's; fit: more
+ * than so many bytes are taken not to fit on the device (the budget is then
+ * halved, down to one atom, and the call ends with LAPW1GPU_ERR_NOMEM if
+ * that is too much), 0 for no such limit.  Frees what is held. */
+int lapw1gpu_test_projection_bytes(lapw1gpu_context* ctx, size_t budget, size_t fit);
+
 /* Page-lock a caller buffer (typically HS, allocated once by INIT_MATRICES,
  * modules.F:526-535) for the context's lifetime, so that the host entry
  * points copy HS at full link speed and overlap those copies with the later

@@ -114,6 +114,64 @@ def test_projection_tiles(ctx, slices, nb, block, lmax):
     assert np.abs(out[1] - out[0]).max() <= (64 * (slices + 1) * 2.0 ** (-7 * slices) + 1e-9) * np.abs(out[0]).max()
 
 
+@pytest.mark.parametrize("slices,nb", [(6, 41), (7, 33)])
+def test_projection_chunks_of_atoms(ctx, slices, nb):
+    """Operands of a few atoms at a time: chunks of one atom, chunks that end
+    inside the type of 17 atoms and span several types, and a budget of which
+    less and less fits.  An atom's sums do not depend on its chunk, so the
+    gradient is the single chunk's up to the order of the atomic sums.  What
+    does not fit at all is an error that leaves the context usable."""
+    p = synth.small_case("manyeq", rkmax=2.5)
+    block, nband = 64, (40 if slices == 6 else 32)
+    nblk = -(-p.nv // block)
+    assert nblk > 2 and p.ndf == 22
+    types = np.repeat(np.arange(p.nat), p.mult)
+    kp_bytes = nblk * block  # one operand row
+    type_bytes = slices * -(-p.ltop ** 2 // 16) * 128 * kp_bytes
+    atom_bytes = slices * 2 * -(-nb // nband) * nband * kp_bytes
+    rng = np.random.default_rng(5)
+    dev = torch.device("cuda", ctx.device)
+    c = torch.from_numpy(rng.standard_normal((nb, p.n)) + 1j * rng.standard_normal((nb, p.n))).to(dev)
+    eps = torch.from_numpy(np.sort(rng.uniform(-1.0, 1.0, nb))).to(dev)
+    occ = torch.from_numpy(rng.uniform(0.0, 2.0, nb)).to(dev)
+    g = torch.empty((p.ndf, 3), dtype=torch.float64, device=dev)
+    kp = ctx.upload(p)
+
+    def gradient(budget, fit=0):
+        ctx.test_projection_bytes(budget, fit)
+        g.fill_(np.nan)
+        torch.cuda.synchronize()
+        kp.forces(c.data_ptr(), p.n, nb, occ.data_ptr(), eps.data_ptr(), g.data_ptr())
+        return g.cpu().numpy(), ctx.last_launches()
+
+    try:
+        ctx.set_precision(lapw1gpu.PREC_SPLIT, 5)
+        ctx.set_force_projection(slices, block)
+        ref, launches = gradient(0)
+        for budget in (1, type_bytes + 5 * atom_bytes, 2 * type_bytes + 8 * atom_bytes):
+            n, a0, a1 = 0, 0, 0  # the chunks' count
+            while a1 < p.ndf:
+                n, a0, a1 = n + 1, a1, a1 + 1
+                while a1 < p.ndf and (types[a1] - types[a0] + 1) * type_bytes + (a1 + 1 - a0) * atom_bytes <= budget:
+                    a1 += 1
+            out, nl = gradient(budget)
+            assert np.abs(out - ref).max() <= 1e-12 * np.abs(ref).max(), budget
+            assert n > 3 and nl == launches + 3 * (n - 1), (budget, n)
+        exps = 4 * 2 * -(-p.ltop ** 2 // 16) * 128 * nblk  # two types' exponents
+        out, nl = gradient(0, 2 * type_bytes + 8 * atom_bytes + exps)
+        assert np.abs(out - ref).max() <= 1e-12 * np.abs(ref).max() and nl > launches
+        with pytest.raises(lapw1gpu.Lapw1GpuError) as e:
+            gradient(0, atom_bytes)
+        assert e.value.code == 2  # LAPW1GPU_ERR_NOMEM
+        out, nl = gradient(0)
+        assert np.abs(out - ref).max() <= 1e-12 * np.abs(ref).max() and nl == launches
+    finally:
+        ctx.test_projection_bytes()
+        ctx.set_force_projection(-1, 1024)
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+        kp.free()
+
+
 # one writer of HS each: k_spherical, k_lo, the HNS product
 @pytest.mark.parametrize("field,lo,stages", [("e", (), 1), ("alo", (0, 1), 1), ("tns", (), 3)])
 @pytest.mark.parametrize("value", [np.nan, np.inf])
