@@ -157,3 +157,36 @@ def test_c3_forces_match_central_differences(ctx, c3_forces, ac):
     assert abs(fd - gsp[a, c]) * to_cart <= TOL_FD_RY_BOHR, (fd * to_cart, gsp[a, c] * to_cart)
     assert abs(fd - gsp4[a, c]) * to_cart <= TOL_FD_RY_BOHR, (fd * to_cart, gsp4[a, c] * to_cart)
     assert abs(fd - gproj[a, c]) * to_cart <= TOL_FD_RY_BOHR, (fd * to_cart, gproj[a, c] * to_cart)
+
+
+@pytest.mark.gpu
+def test_c3_projection_operands_stay_within_6_gib(ctx):
+    """The projections' operands of all 100 atoms of c3 (5 blocks of 1024
+    rows, 600 bands) are 6.8 GB: the adjoint takes the atoms in pieces that
+    leave at most 6 GiB allocated, and the gradient does not show it."""
+    p, nb = synth.config("c3")[0], 600
+    dev = torch.device("cuda", ctx.device)
+    rng = np.random.default_rng(9)
+    c = torch.from_numpy(rng.standard_normal((nb, p.n)) + 1j * rng.standard_normal((nb, p.n))).to(dev)
+    eps = torch.linspace(-1.0, 1.0, nb, dtype=torch.float64, device=dev)
+    occ = torch.ones(nb, dtype=torch.float64, device=dev)
+    out = []
+    kp = ctx.upload(p)
+    try:
+        ctx.set_precision(lapw1gpu.PREC_SPLIT, 5)
+        ctx.set_force_projection(6, 1024)
+        for budget in (0, 16 << 30, 0):  # (the first call sizes the other buffers)
+            ctx.test_projection_bytes(budget)
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info(dev)[0]
+            g = torch.empty((p.ndf, 3), dtype=torch.float64, device=dev)
+            kp.forces(c.data_ptr(), p.n, nb, occ.data_ptr(), eps.data_ptr(), g.data_ptr())
+            out.append((g.cpu().numpy(), free - torch.cuda.mem_get_info(dev)[0]))
+    finally:
+        ctx.test_projection_bytes()
+        ctx.set_force_projection(-1, 1024)
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+        kp.free()
+    (g0, held0), (g1, held1) = out[1:]
+    assert held0 > 6 << 30 and held1 <= (6 << 30) + (16 << 20), (held0, held1)
+    assert np.abs(g1 - g0).max() <= 1e-12 * np.abs(g0).max()
