@@ -41,6 +41,7 @@
 // block (36% less feed, 8 pairs per epilogue thread by a register split) took
 // the same time and was not kept, nor did row pitches of 64 or 128 bytes help.
 #pragma once
+#include "legendre.cuh"
 
 namespace sphtc {
 
@@ -204,42 +205,9 @@ __device__ __forceinline__ double pow2i(int e) {
   return __hiloint2double((min(max(e, -1023), 1024) + 1023) << 20, 0);  // biased exponent 0: the double 0
 }
 
-// Coefficients of (2l+1) P_l(x) by descending power: x^(l odd) times a
-// polynomial of degree l/2 in x^2, P_l = 2^-l sum_k (-1)^k C(l,k) C(2l-2k,l) x^(l-2k)
-struct LegCoef {
-  double c[SPH_LMAX][(SPH_LMAX + 1) / 2];
-};
-__host__ __device__ constexpr LegCoef leg_make() {
-  LegCoef t{};
-  for (int l = 0; l < SPH_LMAX; l++)
-    for (int k = 0; k <= l / 2; k++) {
-      double v = 1.0;
-      for (int i = 1; i <= k; i++) v = v * (l - k + i) / i;      // C(l,k)
-      double w = 1.0;
-      for (int i = 1; i <= l; i++) w = w * (l - 2 * k + i) / i;  // C(2l-2k,l)
-      double q = (k & 1) ? -v * w : v * w;
-      for (int i = 0; i < l; i++) q *= 0.5;
-      t.c[l][k] = q * (2 * l + 1);
-    }
-  return t;
-}
-template <int l, int N>
-__device__ __forceinline__ void leg_poly(const double (&x)[N], double (&w)[N]) {
-  constexpr LegCoef K = leg_make();
-#pragma unroll
-  for (int u = 0; u < N; u++) {
-    const double t = x[u] * x[u];
-    double p = K.c[l][0];
-#pragma unroll
-    for (int k = 1; k <= l / 2; k++) p = fma(p, t, K.c[l][k]);
-    w[u] = (l & 1) ? p * x[u] : p;
-  }
-}
 // w = (2l+1) P_l(x) of N pairs from the explicit polynomials: independent
 // chains with the coefficients as constant operands, and no values of the
-// orders below l to keep.  Rounding: at most eps sum |c_k|, 1e-12 at l = 12
-// near |x| = 1 and below 2e-13 up to l = 10, under the slice products' error
-// at 5 slices (2e-10).  line: bits of the pairs along one line, which take
+// orders below l to keep.  line: bits of the pairs along one line, which take
 // x P_(l-1) at every order (hamilt.F:250-281), so x^l.
 template <int N>
 __device__ __forceinline__ void leg_weights(int l, const double (&x)[N], unsigned line, double (&w)[N]) {
