@@ -296,11 +296,11 @@ __global__ void __launch_bounds__(Cfg<S>::THREADS, 1)
     k_fsp_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, DevProb P,
                const SphCoef* __restrict__ coef, int a0, int t0, int nblk, int fB, int fBp, int nb, int nbp,
                const int* __restrict__ exA, const int* __restrict__ exC, const double* __restrict__ f,
-               const double* __restrict__ eps, double* __restrict__ F, int* __restrict__ status) {
+               const double* __restrict__ eps, double* __restrict__ F, int* __restrict__ status, int never_wait) {
   using C = Cfg<S>;
   constexpr int N = C::N, STAGES = C::STAGES, HB = C::HB;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t full[STAGES], empty[STAGES], tfull, tempty, accbar;
+  __shared__ uint64_t full[STAGES], empty[STAGES], tfull, tempty, accbar, never;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ double sf[C::NB], sfe[C::NB], red[8][3];
@@ -323,6 +323,7 @@ __global__ void __launch_bounds__(Cfg<S>::THREADS, 1)
     mbar_init(&tfull, 1);
     mbar_init(&tempty, 8);  // one arrival per epilogue warp
     mbar_init(&accbar, 1);
+    mbar_init(&never, 1);  // nothing arrives here (the never_wait test hook)
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -377,6 +378,7 @@ __global__ void __launch_bounds__(Cfg<S>::THREADS, 1)
       auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
         return __all_sync(0xffffffffu, wait_or_abort(bar, parity, &abort_flag));
       };
+      if (never_wait) ok = __all_sync(0xffffffffu, sphtc::never_arrives(&never));
       const uint64_t desc0 = desc_sw64(smem_u32(smem));
       for (int p = 0; p < nblk && ok; p++) {
         if (p > 0) ok = wait(&tempty, (uint32_t)(p - 1) & 1);

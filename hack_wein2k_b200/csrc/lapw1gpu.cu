@@ -135,7 +135,7 @@ struct lapw1gpu_context {
   DevBuf fsp;                          // the spherical projections' int8 operands (fsp_products)
   size_t fsp_budget = L1G_FSP_BYTES;   // bytes they may take,
   size_t test_fsp_fit = SIZE_MAX;      // and (test hook) what an allocation of them may take
-  int test_never_wait = 0; // test hook: the spherical tensor kernel's consumer wait runs out
+  int test_never_wait = 0; // test hook: the wait of k_sph_tc's and k_fsp_gemm's MMA issuer runs out
   int last_launches = 0;   // kernels launched by the last call (a library product counts as one)
   std::map<std::string, DevBuf> bufs;
   std::map<std::string, std::pair<int2*, int>> tiles;  // tile lists per shape (kp_tiles)
@@ -343,6 +343,14 @@ static int read_status(lapw1gpu_context* c, cudaStream_t s, int* out, int* nl = 
   CK(cudaStreamSynchronize(s));
   *out = h;
   return LAPW1GPU_OK;
+}
+
+// the return code of a status word (a timed-out wait leaves elements
+// unwritten, which later finite checks see)
+static int status_code(int st) {
+  if (st & L1G_STATUS_TIMEOUT) return LAPW1GPU_ERR_TIMEOUT;
+  if (st & L1G_STATUS_NONFINITE) return LAPW1GPU_ERR_NONFINITE;
+  return st ? LAPW1GPU_ERR_RANGE : LAPW1GPU_OK;
 }
 
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
@@ -1420,9 +1428,7 @@ int lapw1gpu_kpoint_run(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, dou
     c->last_launches = nl;
     c->last_status = hstat;
     fill_stats(c, k, nl, st);
-    if (hstat & L1G_STATUS_TIMEOUT) return LAPW1GPU_ERR_TIMEOUT;
-    if (hstat & L1G_STATUS_NONFINITE) return LAPW1GPU_ERR_NONFINITE;
-    if (hstat) return LAPW1GPU_ERR_RANGE;
+    return status_code(hstat);
   }
   return LAPW1GPU_OK;
 }
@@ -1532,11 +1538,7 @@ int lapw1gpu_setup_batch(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int n
     st->kernel_launches = nl;
     st->ms_host = host_ms;
   }
-  // a timed-out wait leaves elements unwritten, which later finite checks see
-  if (hstat & L1G_STATUS_TIMEOUT) return LAPW1GPU_ERR_TIMEOUT;
-  if (hstat & L1G_STATUS_NONFINITE) return LAPW1GPU_ERR_NONFINITE;
-  if (hstat) return LAPW1GPU_ERR_RANGE;
-  return LAPW1GPU_OK;
+  return status_code(hstat);
 }
 
 int lapw1gpu_get_tuning(lapw1gpu_context* c, lapw1gpu_tuning* t) {
@@ -1819,11 +1821,7 @@ static int setup_host_impl(lapw1gpu_context* c, const lapw1gpu_problem* p, int s
   }
   lapw1gpu_kpoint_free(k);
   if (rc) return rc;
-  // a timed-out wait leaves elements unwritten, which later finite checks see
-  if (hstat & L1G_STATUS_TIMEOUT) return LAPW1GPU_ERR_TIMEOUT;
-  if (hstat & L1G_STATUS_NONFINITE) return LAPW1GPU_ERR_NONFINITE;
-  if (hstat) return LAPW1GPU_ERR_RANGE;
-  return LAPW1GPU_OK;
+  return status_code(hstat);
 }
 
 int lapw1gpu_setup_stages(lapw1gpu_context* c, const lapw1gpu_problem* p, int stages, double* hs, int ldhs,
@@ -1857,11 +1855,7 @@ int lapw1gpu_setup_wait(lapw1gpu_context* c, lapw1gpu_stats* st) {
   c->async_k = nullptr;
   c->async_pending = false;
   if (rc) return rc;
-  // a timed-out wait leaves elements unwritten, which later finite checks see
-  if (hstat & L1G_STATUS_TIMEOUT) return LAPW1GPU_ERR_TIMEOUT;
-  if (hstat & L1G_STATUS_NONFINITE) return LAPW1GPU_ERR_NONFINITE;
-  if (hstat) return LAPW1GPU_ERR_RANGE;
-  return LAPW1GPU_OK;
+  return status_code(hstat);
 }
 
 // hns.F:317-380 sums over LMSORT's grouping of the gaunt list
@@ -2003,7 +1997,8 @@ static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& 
     CUtensorMap ta, tb;
     if (l1g_tmap_3d(&ta, A, Kp, rowsA, S, 128) || l1g_tmap_3d(&tb, B, Kp, rowsB, S, Cf::N)) return LAPW1GPU_ERR_CUDA;
     fsptc::k_fsp_gemm<S><<<dim3(BT, MT, na), Cf::THREADS, Cf::SMEM, s>>>(
-        ta, tb, P, coef, a0, t0, nblk, fB, fBp, nb, nbp, exA, exC, d_occ, d_eps, d_grad, c->d_status);
+        ta, tb, P, coef, a0, t0, nblk, fB, fBp, nb, nbp, exA, exC, d_occ, d_eps, d_grad, c->d_status,
+        c->test_never_wait);
     *nl += 3;
     if (int rc = l1g_launch_status(__FILE__, __LINE__)) return rc;
     if (timed) {
@@ -2295,7 +2290,7 @@ int lapw1gpu_forces(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double* d_c, 
     }
   }
   cudaGetLastError();
-  return hstat ? LAPW1GPU_ERR_RANGE : LAPW1GPU_OK;
+  return status_code(hstat);
 }
 
 // The adjoint of a k-point list queued back to back on the context's stream
@@ -2329,7 +2324,7 @@ int lapw1gpu_forces_batch(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int 
     cudaEventElapsedTime(&t, c->ev[0], c->ev[6]);
     *ms_total = t;
   }
-  return hstat ? LAPW1GPU_ERR_RANGE : LAPW1GPU_OK;
+  return status_code(hstat);
 }
 
 }  // extern "C"

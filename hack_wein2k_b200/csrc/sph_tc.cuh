@@ -324,6 +324,16 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, co
   return true;
 }
 
+// test hook: a wait on a barrier that nothing arrives at, with a short bound
+// (about half a millisecond): false, and the caller takes its timeout path (the
+// other roles' waits keep their full bound)
+__device__ __forceinline__ bool never_arrives(uint64_t* bar) {
+  const long long t0 = clock64();
+  bool in_time = true;
+  while (in_time && !mbar_try_wait(bar, 0)) in_time = clock64() - t0 <= (1LL << 20);
+  return in_time;
+}
+
 // Position in a ring of N slots: the slot and the parity of the current
 // round's completion (counters and divisions would cost the issuing warps
 // more than an MMA)
@@ -437,15 +447,7 @@ __global__ void __launch_bounds__(Cfg<S, KB>::THREADS, 1)
       auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
         return __all_sync(0xffffffffu, wait_or_abort(bar, parity, &abort_flag));
       };
-      if (never_wait) {
-        // test hook: the consumer waits on a barrier that nothing arrives
-        // at, with a short bound (about half a millisecond), and takes the
-        // timeout path below (the other roles' waits keep their full bound)
-        const long long t0 = clock64();
-        bool in_time = true;
-        while (in_time && !mbar_try_wait(&never, 0)) in_time = clock64() - t0 <= (1LL << 20);
-        ok = __all_sync(0xffffffffu, in_time);
-      }
+      if (never_wait) ok = __all_sync(0xffffffffu, never_arrives(&never));
       const uint64_t desc0 = desc_kblock<KB>(smem_u32(smem));
       for (int t = blockIdx.x; t < ntile && ok; t += gridDim.x) {
         for (int l = 0; l < L && ok; l++) {

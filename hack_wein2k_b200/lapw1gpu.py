@@ -222,8 +222,9 @@ class Context:
         return int(self.lib.lapw1gpu_last_launches(self.h))
 
     def test_wait_timeout(self, on: bool) -> None:
-        """Test hook (lapw1gpu_test_wait_timeout): make the spherical tensor
-        kernel's consumer wait run out on later split-precision runs."""
+        """Test hook (lapw1gpu_test_wait_timeout): make the MMA issuer's
+        wait of the spherical tensor kernels run out on later split-precision
+        setups and adjoints."""
         _check("lapw1gpu_test_wait_timeout", self.lib.lapw1gpu_test_wait_timeout(self.h, 1 if on else 0))
 
     def test_projection_bytes(self, budget: int = 0, fit: int = 0) -> None:

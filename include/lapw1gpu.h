@@ -245,8 +245,9 @@ void* lapw1gpu_stream(lapw1gpu_context* ctx);
 
 /* Test hook of the bounded device waits.  No counterpart in the reference.
  * With on = 1, later runs of the split-precision spherical tensor-core
- * kernel make its MMA issuer wait on a barrier that nothing arrives at,
- * bounded to about half a millisecond: the kernel takes its timeout path
+ * kernels (the setup's and the adjoint's projections) make their MMA issuer
+ * wait on a barrier that nothing arrives at, bounded to about half a
+ * millisecond: the kernel takes its timeout path
  * (status bit, copies in flight drained, TMEM freed) and the run returns
  * LAPW1GPU_ERR_TIMEOUT with the context still usable.  on = 0 (the
  * default) restores normal runs. */
@@ -388,7 +389,8 @@ int lapw1gpu_autotune(lapw1gpu_context* ctx, lapw1gpu_kpoint* kp, double* d_hs,
  * fixed.  No counterpart in lapw1 (it has no derivative code); the
  * reference's forces are lapw2's (SRC_lapw2/fomai1.f, l2main.F:630-634) on
  * another formulation.  Problems with HORB potentials (natorb > 0) return
- * LAPW1GPU_ERR_ARG.  Synchronous. */
+ * LAPW1GPU_ERR_ARG.  A non-finite operand of the split-precision products
+ * returns LAPW1GPU_ERR_NONFINITE.  Synchronous. */
 int lapw1gpu_forces(lapw1gpu_context* ctx, lapw1gpu_kpoint* kp,
                     const double* d_c, int ldc, int nb, const double* d_occ,
                     const double* d_eps, double* d_grad);
