@@ -121,6 +121,32 @@ def test_choice_of_the_k_block_is_kept(ctx):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prec", [lapw1gpu.PREC_FP64, lapw1gpu.PREC_SPLIT])
+@pytest.mark.parametrize("nk", [1, 2, 3, 5])
+def test_batches_around_the_number_of_chains(ctx, prec, nk):
+    """Fewer k-points than the four chains of small k-points (one alone runs as
+    a single call does) and one more than they are."""
+    dev = torch.device("cuda", ctx.device)
+    probs = [synth.small_case(k) for k in ("lo", "orb", "apw", "ins", "lo")][:nk]
+    with lapw1gpu.Context(ctx.device, prec=prec) as c:
+        ref = _single(c, probs, dev)
+        kps = [c.upload(p) for p in probs]
+        hs, hd = _alloc(probs, dev)
+        for call in range(2):
+            for t in hs + hd:
+                t.zero_()
+            torch.cuda.synchronize()
+            c.setup_batch(kps, [h.data_ptr() for h in hs], [p.n for p in probs], [d.data_ptr() for d in hd])
+            for i in range(nk):
+                assert np.array_equal(_host(hs[i]), ref[i][0]), (call, i)
+                assert np.array_equal(hd[i].cpu().numpy(), ref[i][1]), (call, i)
+        t = c.autotune(kps[0], hs[0].data_ptr(), probs[0].n, hd[0].data_ptr())
+        assert t["batch_sets"] == 4 and c.tuning()["batch_sets"] == 0
+        for k in kps:
+            k.free()
+
+
+@pytest.mark.gpu
 def test_batch_against_oracle(ctx):
     dev = torch.device("cuda", ctx.device)
     ctx.set_precision(lapw1gpu.PREC_FP64)
