@@ -258,6 +258,8 @@ __device__ __forceinline__ int pr_lane_i(int lane) { return ((lane >> 1) & 1) | 
 // types per staged chunk: as many as the shared memory holds twice
 __host__ __device__ constexpr int pr_tc(int lt) { return lt <= PR_LT ? 5 : 4; }
 
+// 16-byte global -> shared copy that bypasses registers (cp.async), so that
+// a block's staging has all its loads in flight at once
 __device__ __forceinline__ void pr_cp16(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
@@ -736,16 +738,6 @@ __global__ void k_hns_alm(DevProb P, const LoRange* __restrict__ lor, int nlor, 
   }
 }
 
-// 16-byte global -> shared copy that bypasses registers (cp.async), so that
-// a block's staging has all its loads in flight at once
-__device__ __forceinline__ void l1g_cp16(void* dst, const void* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void l1g_cp_wait_all() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
 
 // c += a b for one 8 x 8 tile and 4 k: lane holds a(lane / 4, lane % 4),
 // b(lane % 4, lane / 4), c(lane / 4, 2 (lane % 4) + {0, 1})
@@ -792,16 +784,17 @@ __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int n
         const int row = idx / K, col = idx % K;
         const int ro = row / nsl2, la = row % nsl2, r = col / nsl2, b = col % nsl2;
         const int blk = ro == 0 ? (r == 0 ? 0 : 1) : (r == 0 ? 3 : 4);  // TUU TDU / TUD TDD
-        l1g_cp16(&sM[row * TMUL_MS + col], &T[((size_t)blk * L1G_NSL2 + la) * L1G_NSL2 + b]);
+        pr_cp16(&sM[row * TMUL_MS + col], &T[((size_t)blk * L1G_NSL2 + la) * L1G_NSL2 + b]);
       }
       staged = a;
     }
     const double2* R = Rop + (size_t)a * K * npad;
     for (int idx = tid; idx < K * TMUL_I; idx += 32 * TMUL_WARPS) {
       const int k = idx / TMUL_I, c = idx % TMUL_I;  // npad is a multiple of 64
-      l1g_cp16(&sR[k * TMUL_RS + c], &R[(size_t)k * npad + i0 + c]);
+      pr_cp16(&sR[k * TMUL_RS + c], &R[(size_t)k * npad + i0 + c]);
     }
-    l1g_cp_wait_all();
+    pr_commit();
+    pr_wait<0>();
     __syncthreads();
     double re[TMUL_MF][2][2], im[TMUL_MF][2][2];
 #pragma unroll

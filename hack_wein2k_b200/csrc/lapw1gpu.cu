@@ -86,7 +86,7 @@ struct lapw1gpu_context {
   cudaEvent_t fev[7] = {};  // the last forces call: start, density matrices, k_force_sph, LO columns, end;
                             // [6] the end of the spherical projections
   float fms[7] = {};        // its intervals (ms), read by lapw1gpu_forces_stats; [5] the projections,
-                            // [6] their products (the split_rect_gemm calls)
+                            // [6] their operands and products (per chunk of atoms)
   bool fproj_last = false;  // the last forces call formed spherical projections
   std::vector<cudaEvent_t> fpev;  // timed forces call: around each chunk of the projections
   int fpev_used = 0;
@@ -122,7 +122,7 @@ struct lapw1gpu_context {
   int slices_fsp = -1;   // and of its spherical projections (0: the FP64 pair kernel for every pair;
                          // -1: L1G_FSP_SLICES slices when NV spans L1G_FSP_MIN_BLOCKS blocks)
   int fsp_block = 1024;  // PW rows per block of the spherical projections
-  cublasHandle_t blas[L1G_MAX_SETS] = {};  // library ZGEMMs, one handle (and workspace) per scratch set
+  cublasHandle_t blas = nullptr;            // the FP64 adjoint's library ZGEMMs
   cusolverDnHandle_t solver = nullptr;      // the eigen-solve (lapw1gpu_seclr4)
   // tunables (lapw1gpu_autotune)
   int hns_diag_b = 512;    // kept for callers that set it; the FP64 HNS update is one product without blocks
@@ -233,10 +233,10 @@ struct lapw1gpu_context {
   void* sbuf(int set, const char* name, size_t bytes) {
     return set == 0 ? buf(name, bytes) : buf(std::string(name) + "#" + std::to_string(set), bytes);
   }
-  cublasHandle_t handle(int set, cudaStream_t s) {
-    if (!blas[set] && cublasCreate(&blas[set]) != CUBLAS_STATUS_SUCCESS) return nullptr;
-    if (cublasSetStream(blas[set], s) != CUBLAS_STATUS_SUCCESS) return nullptr;
-    return blas[set];
+  cublasHandle_t handle(cudaStream_t s) {
+    if (!blas && cublasCreate(&blas) != CUBLAS_STATUS_SUCCESS) return nullptr;
+    if (cublasSetStream(blas, s) != CUBLAS_STATUS_SUCCESS) return nullptr;
+    return blas;
   }
   void drop_graphs() {
     for (auto& g : graphs)
@@ -480,8 +480,7 @@ int lapw1gpu_finalize(lapw1gpu_context* c) {
   cudaDeviceSynchronize();
   for (void* h : c->host_pinned) cudaHostUnregister(h);
   c->drop_graphs();
-  for (auto& h : c->blas)
-    if (h) cublasDestroy(h);
+  if (c->blas) cublasDestroy(c->blas);
   if (c->solver) cusolverDnDestroy(c->solver);
   for (auto& kv : c->bufs)
     if (kv.second.ptr) cudaFree(kv.second.ptr);
@@ -563,7 +562,7 @@ int lapw1gpu_forces_stats(lapw1gpu_context* c, lapw1gpu_stats* st) {
   st->ms_albl = c->fms[0];      // operands and the density matrices
   st->ms_spherical = c->fms[1] + c->fms[2];
   st->ms_sph_main = c->fms[2] - c->fms[5];  // k_force_sph
-  st->ms_sph_slice = c->fms[6];               // the products of the spherical projections
+  st->ms_sph_slice = c->fms[6];               // the spherical projections' operands and products
   st->ms_table = c->fms[5] - c->fms[6];       // and their other kernels (harmonics, exponents, bins)
   st->ms_lo = c->fms[3];        // the step-function sums and the LO columns
   st->ms_hns = c->fms[4];       // the HNS part
@@ -1479,8 +1478,7 @@ int lapw1gpu_setup_batch(lapw1gpu_context* c, lapw1gpu_kpoint* const* kps, int n
     if (!kps[i] || kps[i]->ctx != c || !d_hs[i] || !d_hsdiag[i] || ldhs[i] < kps[i]->n) return LAPW1GPU_ERR_ARG;
   CK(cudaSetDevice(c->device));
   std::vector<uintptr_t> key = {(uintptr_t)nk,         (uintptr_t)stages,        (uintptr_t)c->prec,
-                                (uintptr_t)(c->slices * 16 + c->slices_hns), (uintptr_t)c->hns_diag_b,
-                                (uintptr_t)c->split_group,
+                                (uintptr_t)(c->slices * 16 + c->slices_hns), (uintptr_t)c->split_group,
                                 (uintptr_t)c->sph_tc,  (uintptr_t)c->sph_kb,
                                 (uintptr_t)batch_chains(c, kps, nk),
                                 (uintptr_t)c->test_never_wait};
@@ -2046,8 +2044,9 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
   double2* rhoe = (double2*)c->buf("frc_rhoe", sizeof(double2) * (size_t)n * n);
   SphCoef* coef = (SphCoef*)c->buf("coef", sizeof(SphCoef) * nat * ltop);
   if (!P.al || !P.bl || !P.phase || !Cf || !Ce || !rho || !rhoe || !coef) return LAPW1GPU_ERR_NOMEM;
-  cublasHandle_t h = c->handle(0, s);
-  if (!h) return LAPW1GPU_ERR_CUDA;
+  const bool split_rho = c->prec == LAPW1GPU_PREC_SPLIT;
+  cublasHandle_t h = split_rho ? nullptr : c->handle(s);  // FP64: the HNS projections
+  if (!h && !split_rho) return LAPW1GPU_ERR_CUDA;
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0), zero = make_cuDoubleComplex(0.0, 0.0);
   int nlf = 0;  // kernels launched (a library product counts as one)
   if (timed) CK(cudaEventRecord(c->fev[0], s));
@@ -2055,7 +2054,6 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
   k_albl<<<dim3((k->nvpad + 127) / 128, nat), 128, 0, s>>>(P, c->d_status);
   k_phase<<<dim3((k->npad + 127) / 128, ndf), 128, 0, s>>>(P);
   k_sph_coef<<<nat, 32, 0, s>>>(P, coef);
-  const bool split_rho = c->prec == LAPW1GPU_PREC_SPLIT;
   k_force_weight<<<dim3((n + 127) / 128, nb), 128, 0, s>>>(n, nb, C, ldc, d_occ, d_eps, Cf, Ce);
   nlf += 4;  // k_albl, k_phase, k_sph_coef, k_force_weight
   CK(cudaGetLastError());
@@ -2396,7 +2394,7 @@ extern "C" int lapw1gpu_seclr4(lapw1gpu_context* c, const double* d_hs_, int ldh
 // pool (and cudaFree synchronises the device under their stream work).
 // This entry point computes the same HNS update as the HNS stage of
 // lapw1gpu_setup_stages, with all of its intermediate buffers (the uploaded
-// inputs, AL/BL, phases, the HNS operands, tile list, status word) carved
+// inputs, AL/BL, phases, the HNS operands, status word) carved
 // from one file-scope device array of L1G_NOALLOC_BYTES.  Every GPU that
 // loads the library holds that array until the process exits.
 // ---------------------------------------------------------------------

@@ -190,8 +190,9 @@ def test_autotune_keeps_results_exact(ctx, prec, slices):
     p = synth.small_case("lo", rkmax=6.0)
     kp = ctx.upload(p)
     hs, hd = _alloc([p], dev)
+    ctx.set_tuning(hns_diag_b=256)
     t = ctx.autotune(kp, hs[0].data_ptr(), p.n, hd[0].data_ptr())
-    assert t["hns_diag_b"] in (256, 512, 1024, 2048)
+    assert t["hns_diag_b"] == 256  # without effect, kept as it was set
     assert t["split_group"] in (4, 8, 16, 32) and t["sph_tc"] in (0, 1) and t["ms_best"] > 0
     assert t["sph_kblock"] in (64, 128)
     kp.run(hs[0].data_ptr(), p.n, hd[0].data_ptr(), stats=True)

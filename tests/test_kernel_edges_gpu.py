@@ -33,7 +33,8 @@ def _check(ctx, p, tol):
 
 
 # 32- and 64-row tiles of k_spherical and k_tri_gemm; 1537 rows take the
-# 64-wide product tiles (300 of them), 1472 the 32-wide ones
+# 64-wide product tiles (25 tile rows, 325 tiles: at least two per SM), 1472
+# (23, 276) the 32-wide ones
 @pytest.mark.parametrize("nv", [1, 31, 32, 33, 63, 64, 65, 97, 1472, 1537])
 def test_fp64_row_counts(ctx, nv):
     ctx.set_precision(lapw1gpu.PREC_FP64)
