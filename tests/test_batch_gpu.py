@@ -121,6 +121,26 @@ def test_choice_of_the_k_block_is_kept(ctx):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind,rkmax,kb,chains", [("lo", 5.0, 64, 4), ("lo", 12.0, 64, 2), ("manyeq", 2.5, 128, 4)])
+def test_rules_where_nothing_is_chosen(ctx, kind, rkmax, kb, chains):
+    """What runs where the caller chose no K block and no chains, as the
+    autotuner reports it in FP64, which tunes neither: 64-byte blocks where
+    they pad K = 2 roundup(2 atoms, 16) bytes less (3 atoms: 32 bytes; 22
+    atoms: 96, either block pads to 128), four chains up to N = 1088."""
+    p = synth.small_case(kind, rkmax=rkmax)
+    assert (p.n <= 1088) == (chains == 4)
+    dev = torch.device("cuda", ctx.device)
+    with lapw1gpu.Context(ctx.device) as c:
+        kp = c.upload(p)
+        hs, hd = _alloc([p], dev)
+        torch.cuda.synchronize()
+        t = c.autotune(kp, hs[0].data_ptr(), p.n, hd[0].data_ptr())
+        kp.free()
+        assert (t["sph_kblock"], t["batch_sets"]) == (kb, chains)
+        assert c.tuning()["sph_kblock"] == 0 and c.tuning()["batch_sets"] == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("prec", [lapw1gpu.PREC_FP64, lapw1gpu.PREC_SPLIT])
 @pytest.mark.parametrize("nk", [1, 2, 3, 5])
 def test_batches_around_the_number_of_chains(ctx, prec, nk):

@@ -173,6 +173,39 @@ def test_projection_chunks_of_atoms(ctx, slices, nb):
         kp.free()
 
 
+@pytest.mark.parametrize("pin", [False, True])
+def test_upload_is_done_with_the_callers_arrays(ctx, pin):
+    """Arrays of up to 256 KiB go through the context's staging buffer, longer
+    ones (the T blocks of six types and of four, 540 and 360 KB) straight from
+    the caller's memory, page-locked or not.  Once upload returns, the caller
+    may overwrite either: the k-points still give what they held, also after
+    another upload has used the staging buffer."""
+    dev = torch.device("cuda", ctx.device)
+    ctx.set_precision(lapw1gpu.PREC_FP64)
+    four = synth.Cell("P", (12.0, 12.0, 12.0), (90.0, 90.0, 90.0),
+                      [dict(pos=[[0.25 * q, 0.3 * q, 0.2 * q]], rmt=1.2) for q in range(4)])
+    probs = [synth.small_case("manyeq", rkmax=2.5), synth.synth_problem(four, 2.6, (0.1, 0.2, 0.3), seed=4)]
+    want = [ctx.setup(p) for p in probs]
+    kps = []
+    for p in probs:
+        mine = {}
+        for name in ("tns", "warp", "kzz", "xk", "p", "pos"):
+            a = np.ascontiguousarray(getattr(p, name))
+            t = torch.empty(a.nbytes, dtype=torch.uint8, pin_memory=pin)
+            mine[name] = t.numpy().view(a.dtype).reshape(a.shape)
+            mine[name][...] = a
+        assert mine["tns"].nbytes > 256 << 10 > mine["xk"].nbytes
+        kps.append(ctx.upload(p.copy(**mine)))
+        for a in mine.values():
+            a.view(np.uint8)[...] = 0xff  # NaN, or -1
+    for p, kp, (hs, hd) in zip(probs, kps, want):
+        d_hs = torch.empty((p.n, p.n), dtype=torch.complex128, device=dev)
+        d_hd = torch.empty(p.n, dtype=torch.complex128, device=dev)
+        kp.run(d_hs.data_ptr(), p.n, d_hd.data_ptr(), stats=True)
+        assert np.array_equal(d_hs.cpu().numpy().T, hs) and np.array_equal(d_hd.cpu().numpy(), hd)
+        kp.free()
+
+
 # one writer of HS each: k_spherical, k_lo, the HNS product
 @pytest.mark.parametrize("field,lo,stages", [("e", (), 1), ("alo", (0, 1), 1), ("tns", (), 3)])
 @pytest.mark.parametrize("value", [np.nan, np.inf])
