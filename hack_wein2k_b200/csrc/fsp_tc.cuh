@@ -23,7 +23,8 @@
 // block.  Only the epilogue's TMEM reads stall the MMAs (the next block needs
 // the same accumulators); the contraction runs beside the next block's.
 // Measured at 100 atoms, NV = 11777, 400 bands, 6 slices, blocks of 1024 rows:
-// products 15.1 ms (3.0e15 int8 ops/s with the padding), operands 3.7 and 2.5;
+// products 15.4 ms (2.9e15 int8 ops/s with the padding; tensor pipe active 64%
+// of the time), operands 3.7 and 2.5, in three pieces of atoms;
 // the complex products over blocks, their slicing, k-major left operand and
 // prefix kernel before took 38.  The operands are bound by the integer work of
 // cutting 1.7e9 values into 6 digits (2.1 TB/s of stores).

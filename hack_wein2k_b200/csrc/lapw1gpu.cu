@@ -1101,8 +1101,8 @@ static bool sph_tc_supported(int S) { return S >= 4 && S <= 7; }
 
 // 128-byte K blocks in k_sph_tc, for K = Kp bytes per row?  They fit two stages
 // up to 5 slices.  Where no value was chosen: 64-byte blocks when they pad K
-// less (the rest of the last block is fed as zeros): K = 160 1.37 ms against
-// 1.44 (40 atoms), K = 416 21.1 against 23.0 (100 atoms); at equal padding the
+// less (the rest of the last block is fed as zeros): K = 160 1.33 ms against
+// 1.42 (40 atoms), K = 416 21.6 against 23.2 (100 atoms); at equal padding the
 // halved count of blocks is up to 2.5% faster (K = 256: 1.59 against 1.62).
 static bool sph_kb128(const lapw1gpu_context* c, int Kp) {
   if (c->slices > 5) return false;
@@ -1435,9 +1435,16 @@ int lapw1gpu_kpoint_run(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, dou
 // ---- k-point batches: one captured graph per argument set ----
 // Concurrent chains of a batch where the caller chose none: a k-point of up
 // to L1G_SMALL_N rows leaves most SMs idle in most of its kernels (fewer than
-// four 32 x 32 pair tiles per SM), so its batch runs on every chain there is (16
-// k-points of N = 704, FP64: 1.10 ms on four chains, 1.59 on two); larger ones on
-// two (four k-points of N = 4950: kernels that fill the SMs anyway).
+// four 32 x 32 pair tiles per SM), so its batch runs on every chain there is.
+// Above it what four chains gain over two falls, and two more scratch sets (HNS
+// operands: 16 bytes x 50 per atom x N each for L and R, split ones with their
+// slices) are kept for it.  Eight k-points (four from N = 3214), two chains
+// against four, FP64 and split, ms:
+//   N   92  0.296 0.163   0.445 0.250     N 1102  1.89  1.60   1.30 1.11
+//   N  369  0.403 0.235   0.537 0.341     N 1622  4.69  4.16   2.23 2.05
+//   N  705  0.704 0.514   0.786 0.580     N 2418 11.50 11.05   4.66 4.40
+//   N 1059  1.459 1.220   1.184 1.009     N 3214 12.79 12.47   4.30 4.13
+//                                         N 4283 28.45 27.85   8.47 8.51
 #define L1G_SMALL_N 1088
 static int chains_for(const lapw1gpu_context* c, int n) {
   if (c->batch_sets) return c->batch_sets;

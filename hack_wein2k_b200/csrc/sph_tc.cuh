@@ -27,19 +27,20 @@
 // mbarrier wait is bounded; a timeout sets a status bit and ends the CTA's
 // work cleanly (copies drained, MMAs complete, TMEM freed).
 //
-// What bounds it (clock sums of the roles, 5 slices): at 100 atoms (13 K steps
-// per l) the tensor core, about 60% of the kernel, and the operand feed that
-// it waits for the rest of the time; at 40 atoms (5 K steps) MMAs, feed and
-// epilogue about equally.  Issued by one lane in a branch of its own, an MMA
+// What bounds it, by the MMA issuer's clocks (5 slices, 64-byte K blocks): at
+// 100 atoms (13 K steps per l) 66% in issuing, behind the tensor core's queue,
+// 29% in waits for operands, 5% for a free accumulator; at 40 atoms (5 K steps)
+// 53, 21 and 26%.  The tensor pipe is active 53 and 39% of the time.  Issued by one lane in a branch of its own, an MMA
 // took 110 clocks of that lane against 77 on the tensor core, and the scales
 // of the epilogue (Legendre weight, exponents) 580 clocks per pair and l
 // behind the TMEM loads; with the issue from a converged warp, the scales
 // formed before the wait for the accumulator, explicit polynomials and the
-// tile's rows in shared memory, 40 atoms (N = 4937) went from 1.69 to 1.37 ms
-// and 100 atoms (N = 12677) from 22.0 to 19.4 ms (38.0 to 33.1 Mclk; the power
-// cap then lowers the clock).  A tile of two 12-I halves that share each A
+// tile's rows in shared memory, 40 atoms (N = 4937) went from 1.69 to 1.33 ms
+// and 100 atoms (N = 12677) from 38.0 to 30.2 Mclk, 22.0 to 20.4-21.6 ms: the
+// power cap sets the clock there.  A tile of two 12-I halves that share each A
 // block (36% less feed, 8 pairs per epilogue thread by a register split) took
-// the same time and was not kept, nor did row pitches of 64 or 128 bytes help.
+// the same time and was not kept (which of the shares grew instead was not
+// recorded), nor did row pitches of 64 or 128 bytes help.
 #pragma once
 #include "legendre.cuh"
 

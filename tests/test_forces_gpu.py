@@ -48,7 +48,7 @@ def test_adjoint_matches_oracle_hellmann_feynman(ctx, kind):
 def test_split_density_matrices_match_fp64(ctx, kind):
     """In split precision lapw1gpu_forces forms rho and rhoE as int8 slice
     products (5 slices); for the same eigenvectors the gradient agrees with
-    the FP64 one (ZHERKX density matrices) to 1e-8 of its largest component."""
+    the FP64 one (k_tri_gemm density matrices) to 1e-8 of its largest component."""
     p = synth.small_case(kind)
     w, _ = FR.eigh(p)
     nb, _ = FR.gapped_nb(w)

@@ -1,5 +1,6 @@
 """The algebra behind the adjoint's spherical projections (forces.cuh:
-frc_zlm, k_force_rsph, k_force_pre), restated in numpy on seeded inputs.
+frc_zlm; fsp_tc.cuh: the operands' product and k_fsp_gemm's contraction with
+the prefix), restated in numpy on seeded inputs.
 
   * the real harmonics of frc_zlm's recursion (Q_mm = (2m-1)!!, the
     three-term recursion in l, sqrt((2l+1)(l-m)!/(l+m)!), sqrt 2 and
@@ -122,7 +123,8 @@ def _pair_sum(c, pairs):
 
 
 def _projections(c, rows):
-    """Y[a, alpha, lm, g, b] over `rows`: the product of k_force_rsph's operand with (G c)^T."""
+    """Y[a, alpha, lm, g, b] over `rows`: A^alpha Z_lm {1, kappa_g} times conj(phase_a) c_b (k_fsp_left,
+    k_fsp_right), summed over the rows."""
     kv = c["kv"]
     rk = np.linalg.norm(kv, axis=1)
     Z = np.array([zlm(kv[i] / rk[i] if rk[i] > 0 else np.array([0.0, 0.0, 1.0])) for i in rows])
@@ -138,7 +140,7 @@ def _projections(c, rows):
 
 
 def _contract(c, Pre, Y):
-    """k_force_pre's sum for one block against the prefix."""
+    """k_fsp_gemm's sum for one block against the prefix."""
     cf = c["coef"]
     lofm = np.concatenate([[l] * (2 * l + 1) for l in range(LT)])
     F = np.zeros((c["ndf"], 3))
