@@ -846,11 +846,14 @@ __global__ void __launch_bounds__(32 * TMUL_WARPS, 2) k_hns_tmul(int npad, int n
 // 62 and 70 us at 100 atoms, where it runs beside the spherical stage.  A row has ALM, BLM, CLM on the atoms of its own type only, and
 // there only at its own l: the sums run over the non-zero b (bits of a ballot;
 // NaN counts as non-zero), 1 + 3 + 5 of 25 for s, p and d rows, and a row
-// that is zero on the atom writes C2 = 0 and leaves L as it is.
+// that is zero on the atom writes C2 = 0 and leaves L as it is.  A non-finite T
+// entry that meets zeros only is reported all the same: with a zero it makes
+// the full sums, and so HS, NaN.  The first block of each type looks.
 #define LOOPS_ROWS 8
 __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __restrict__ tns,
                                                     double2* __restrict__ Lop, const double2* __restrict__ Rop,
-                                                    const double2* __restrict__ Clo, double2* __restrict__ C2lo) {
+                                                    const double2* __restrict__ Clo, double2* __restrict__ C2lo,
+                                                    int* __restrict__ status) {
   __shared__ double2 sX[LOOPS_ROWS][3][L1G_NSL2];
   const int la = threadIdx.x, cy = threadIdx.y;
   const int c0 = blockIdx.x * LOOPS_ROWS;  // first LO row of the block
@@ -869,6 +872,16 @@ __global__ void __launch_bounds__(256) k_hns_lo_ops(DevProb P, const double2* __
         v = Clo[((size_t)a * nsl2 + b) * P.nlo + cc];
     }
     sX[r][w][b] = v;
+  }
+  if (blockIdx.x == 0 && a == P.afirst[P.atype[a]]) {
+    const double2* Ta = tns + (size_t)P.atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2;
+    bool bad = false;
+    for (int q = threadIdx.y * 32 + threadIdx.x; q < 5 * nsl2 * nsl2; q += 256) {
+      const int w = q / (nsl2 * nsl2), lb = q % (nsl2 * nsl2);
+      const int blk = w == 0 ? 2 : w + 4;  // TUU21; TUD21, TUU12, TDU12, TUU22
+      bad |= l1g_nonfinite(__ldg(Ta + ((size_t)blk * L1G_NSL2 + lb / nsl2) * L1G_NSL2 + lb % nsl2));
+    }
+    if (bad) atomicOr(status, L1G_STATUS_NONFINITE);
   }
   __syncthreads();
   const double2* T = tns + (size_t)P.atype[a] * LAPW1GPU_NTNS * L1G_NSL2 * L1G_NSL2 + min(la, nsl2 - 1) * L1G_NSL2;

@@ -940,7 +940,8 @@ static const int2* tiles_tri(lapw1gpu_kpoint* k, const char* name, int n, int T,
 // LO-row terms (k_hns_lo_ops).  Without Lop (the adjoint, which needs R and
 // CLM only) L is not formed.
 static int launch_hns_ops(lapw1gpu_context* c, const DevProb& P, const double2* tns, const LoRange* lor, int nlor,
-                          double2* Lop, double2* Rop, double2* Clo, double2* C2lo, cudaStream_t s, int* nl) {
+                          double2* Lop, double2* Rop, double2* Clo, double2* C2lo, int* status, cudaStream_t s,
+                          int* nl) {
   const int nsl2 = (P.lnsmax + 1) * (P.lnsmax + 1);
   k_hns_alm<<<dim3((P.npad + 127) / 128, P.ndf), 128, 0, s>>>(P, lor, nlor, Rop, Clo);
   if (!Lop) {
@@ -959,7 +960,7 @@ static int launch_hns_ops(lapw1gpu_context* c, const DevProb& P, const double2* 
   *nl += 2;
   if (P.nlo > 0) {
     k_hns_lo_ops<<<dim3((P.nlo + LOOPS_ROWS - 1) / LOOPS_ROWS, P.ndf), dim3(32, 8), 0, s>>>(P, tns, Lop, Rop, Clo,
-                                                                                           C2lo);
+                                                                                           C2lo, status);
     *nl += 1;
   }
   return l1g_launch_status(__FILE__, __LINE__);
@@ -1209,7 +1210,8 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     cudaStream_t a = c->aux[set];
     CK(cudaEventRecord(c->auxf[set], s));
     CK(cudaStreamWaitEvent(a, c->auxf[set], 0));
-    int rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, a, &nl);
+    int rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo,
+                            c->d_status, a, &nl);
     if (!rc && hns_split)
       rc = split_hns_gemm(c, k, set, n, k->npad, Khns, Lop, Rop, d_hs, ldhs, c->slices_hns, a, &nl, nullptr,
                           nullptr, 0, 1);
@@ -1309,7 +1311,8 @@ static int kpoint_run_impl(lapw1gpu_context* c, lapw1gpu_kpoint* k, int stages, 
     if (hns_fork)
       CK(cudaStreamWaitEvent(s, c->auxj[set], 0));
     else
-      rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, s, &nl);
+      rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), Lop, Rop, Clo, C2lo, c->d_status, s,
+                          &nl);
     if (rc) return rc;
     if (hns_split) {
       rc = split_hns_gemm(c, k, set, n, k->npad, K, Lop, Rop, d_hs, ldhs, c->slices_hns, s, &nl, hp,
@@ -2199,8 +2202,8 @@ static int forces_enqueue(lapw1gpu_context* c, lapw1gpu_kpoint* k, const double*
     if (!Rop || !Clo || !Y || !Z) return LAPW1GPU_ERR_NOMEM;
     int nl = 0;
     // R and CLM only: the adjoint applies T to Y = R^H (G c), not L = M conj(R)
-    int rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), nullptr, Rop, Clo, nullptr, s,
-                            &nl);
+    int rc = launch_hns_ops(c, P, k->d_tns, k->d_loranges, (int)k->loranges.size(), nullptr, Rop, Clo, nullptr,
+                            c->d_status, s, &nl);
     if (rc) return rc;
     nlf += nl;
     if ((rc = make_gc(split_rho))) return rc;
@@ -2562,7 +2565,7 @@ extern "C" int lapw1gpu_hns_noalloc(const lapw1gpu_problem* p, double* d_hs_, in
   k_albl<<<dim3((nvpad + 127) / 128, nat), 128, 0, s>>>(P, d_status);
   k_phase<<<dim3((npad + 127) / 128, ndf), 128, 0, s>>>(P);
   int nops = 0;
-  rc = launch_hns_ops(nullptr, P, d_tns, d_lor, nlor, Lop, Rop, Clo, C2lo, s, &nops);
+  rc = launch_hns_ops(nullptr, P, d_tns, d_lor, nlor, Lop, Rop, Clo, C2lo, d_status, s, &nops);
   if (rc) return rc;
   rc = launch_tri(nullptr, n, 0, n, K, Lop, npad, Rop, npad, d_hs, ldhs, 0, nullptr, s, &nops);
   if (!rc && p->nlo > 0)

@@ -206,6 +206,26 @@ def test_upload_is_done_with_the_callers_arrays(ctx, pin):
         kp.free()
 
 
+@pytest.mark.parametrize("prec", [lapw1gpu.PREC_FP64, lapw1gpu.PREC_SPLIT])
+@pytest.mark.parametrize("blk", [2, 5, 6, 7, 8])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_nonfinite_t_entry_of_an_absent_l(ctx, prec, blk, value):
+    """An entry of the local orbitals' T blocks at an l without local orbitals
+    meets zero coefficients only, which make the sums NaN as they stand: the
+    setup reports it."""
+    p = _plain(5.0, lo_l=(0,))
+    tns = np.array(p.tns, copy=True)
+    tns[p.nat - 1, blk, 3, 7] = value  # l = 1, l' = 2
+    ctx.set_precision(prec, 5)
+    try:
+        with pytest.raises(lapw1gpu.Lapw1GpuError) as ei:
+            ctx.setup(p.copy(tns=tns))
+        assert ei.value.code == 4
+        ctx.setup(p)
+    finally:
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+
+
 # one writer of HS each: k_spherical, k_lo, the HNS product
 @pytest.mark.parametrize("field,lo,stages", [("e", (), 1), ("alo", (0, 1), 1), ("tns", (), 3)])
 @pytest.mark.parametrize("value", [np.nan, np.inf])
