@@ -1965,30 +1965,22 @@ static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& 
   const int nv = k->nv, ndf = k->ndf, MT = (k->ltop * k->ltop + fsptc::LMT - 1) / fsptc::LMT;
   const int nblk = (nv + fB - 1) / fB, fBp = round_up(fB, 64), Kp = nblk * fBp;
   const int BT = (nb + Cf::NB - 1) / Cf::NB, nbp = BT * Cf::NB;
-  const size_t typeA = (size_t)S * MT * 128 * Kp, atomB = (size_t)S * 2 * nbp * Kp;
+  const size_t typeA = (size_t)S * MT * 128 * Kp, atomB = (size_t)S * 2 * nbp * Kp;  // multiples of 1024 bytes
   // atoms [at[i], at[i+1]) per chunk; left operands of the types they span
   std::vector<int> at;
-  int8_t *A = nullptr, *B = nullptr;
-  int* exA = nullptr;
+  int8_t* A = nullptr;  // a chunk's left operands, its right ones, the left ones' exponents
   for (size_t budget = c->fsp_budget;;) {
-    size_t needA = 0, needB = 0;
+    size_t need = 0;  // bytes of the largest chunk
     at.assign(1, 0);
     for (int a0 = 0; a0 < ndf;) {
       int a1 = a0 + 1;
       auto bytes = [&](int e) { return (size_t)(k->atype[e - 1] - k->atype[a0] + 1) * typeA + (size_t)(e - a0) * atomB; };
       while (a1 < ndf && bytes(a1 + 1) <= budget) a1++;
-      needA = std::max(needA, (size_t)(k->atype[a1 - 1] - k->atype[a0] + 1));
-      needB = std::max(needB, (size_t)(a1 - a0));
+      need = std::max(need, bytes(a1) + sizeof(int) * (k->atype[a1 - 1] - k->atype[a0] + 1) * MT * 128 * nblk);
       at.push_back(a0 = a1);
     }
-    // A, B (multiples of 1024 bytes) and the exponents of A
-    const size_t need = needA * typeA + needB * atomB + sizeof(int) * needA * MT * 128 * nblk;
     A = (int8_t*)c->fsp_buf(need);
-    if (A) {
-      B = A + needA * typeA;
-      exA = (int*)(B + needB * atomB);
-      break;
-    }
+    if (A) break;
     if ((int)at.size() == ndf + 1) return LAPW1GPU_ERR_NOMEM;  // one atom at a time already
     budget = std::min(budget, need) / 2;
   }
@@ -1996,6 +1988,8 @@ static int fsp_products(lapw1gpu_context* c, lapw1gpu_kpoint* k, const DevProb& 
   for (size_t q = 0; q + 1 < at.size(); q++) {
     const int a0 = at[q], na = at[q + 1] - a0, t0 = k->atype[a0], nt = k->atype[a0 + na - 1] - t0 + 1;
     const size_t rowsA = (size_t)nt * MT * 128, rowsB = (size_t)na * 2 * nbp;
+    int8_t* B = A + nt * typeA;
+    int* exA = (int*)(B + na * atomB);
     if (timed) {
       while (c->fpev.size() < 2 * (q + 1)) {
         cudaEvent_t e;

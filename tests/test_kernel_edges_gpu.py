@@ -149,16 +149,18 @@ def test_projection_chunks_of_atoms(ctx, slices, nb):
         ctx.set_precision(lapw1gpu.PREC_SPLIT, 5)
         ctx.set_force_projection(slices, block)
         ref, launches = gradient(0)
+        exps = 4 * 2 * -(-p.ltop ** 2 // 16) * 128 * nblk
         for budget in (1, type_bytes + 5 * atom_bytes, 2 * type_bytes + 8 * atom_bytes):
             n, a0, a1 = 0, 0, 0  # the chunks' count
             while a1 < p.ndf:
                 n, a0, a1 = n + 1, a1, a1 + 1
                 while a1 < p.ndf and (types[a1] - types[a0] + 1) * type_bytes + (a1 + 1 - a0) * atom_bytes <= budget:
                     a1 += 1
-            out, nl = gradient(budget)
-            assert np.abs(out - ref).max() <= 1e-12 * np.abs(ref).max(), budget
-            assert n > 3 and nl == launches + 3 * (n - 1), (budget, n)
-        exps = 4 * 2 * -(-p.ltop ** 2 // 16) * 128 * nblk  # two types' exponents
+            # (twice: with no more room than the budget and the exponents of two types)
+            for fit in (0, max(budget, type_bytes + atom_bytes) + exps):
+                out, nl = gradient(budget, fit)
+                assert np.abs(out - ref).max() <= 1e-12 * np.abs(ref).max(), budget
+                assert n > 3 and nl == launches + 3 * (n - 1), (budget, n, nl - launches)
         out, nl = gradient(0, 2 * type_bytes + 8 * atom_bytes + exps)
         assert np.abs(out - ref).max() <= 1e-12 * np.abs(ref).max() and nl > launches
         with pytest.raises(lapw1gpu.Lapw1GpuError) as e:
