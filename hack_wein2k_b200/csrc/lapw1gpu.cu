@@ -55,8 +55,9 @@ struct DevBuf {
 #define L1G_MAX_SETS 4  // concurrent k-point chains in a batch (scratch sets)
 #define L1G_MAX_GROUPS 16
 // Default budget of the adjoint's projection operands, which stay allocated.  At
-// 100 atoms they are 13.4 GB in one piece; the whole adjoint takes 45.1 ms so,
-// 45.0 in pieces of 6 GiB (three) and 45.5 of 4 GiB (medians that vary by 1 ms).
+// 100 atoms they are 13.4 GB in one piece; the whole adjoint takes 45.8 ms so
+// and 46.0 in pieces of 6 GiB (47, 47 and 6 atoms; pieces of equal size the same),
+// 0.5 more in pieces of 4 GiB.
 #define L1G_FSP_BYTES (6ull << 30)
 #define L1G_STAGE_MAX (256u << 10)  // an upload's arrays up to this size go through page-locked staging
 
