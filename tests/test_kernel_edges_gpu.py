@@ -5,8 +5,10 @@ import numpy as np
 import pytest
 import torch
 
+from hack_wein2k_b200 import forces as FO
 from hack_wein2k_b200 import lapw1gpu, synth
 from oracle import oracle as O
+from tests import force_ref as FR
 from tests.helpers import rel_errors
 
 TOL_FP64 = 1e-12
@@ -79,6 +81,41 @@ def test_orbital_l(ctx, prec, tol, orb):
         _check(ctx, _plain(5.0, lo_l=(0, 2), apw_l=(1,), rotate_local=True, orb=orb), tol)
     finally:
         ctx.set_precision(lapw1gpu.PREC_FP64)
+
+
+@pytest.fixture(scope="module")
+def many_lo():
+    """17 equivalent atoms of one type and five one-atom types, local orbitals
+    on all: k_lo and k_force_lo hold the Y_lm of eight atoms at a time."""
+    return synth.synth_problem(synth.cell_many_equiv(), 2.2, (0.13, 0.27, 0.41), seed=7, lo_l=(0, 1), rotate_local=True)
+
+
+@pytest.mark.parametrize("prec,tol", [(lapw1gpu.PREC_FP64, TOL_FP64), (lapw1gpu.PREC_SPLIT, TOL_SPLIT[7])])
+@pytest.mark.parametrize("orb", [False, True])
+def test_local_orbitals_of_many_equivalent_atoms(ctx, many_lo, prec, tol, orb):
+    p = many_lo if not orb else synth.synth_problem(synth.cell_many_equiv(), 2.2, (0.13, 0.27, 0.41), seed=7,
+                                                    lo_l=(0, 2), rotate_local=True, orb=((1, (2,)), (3, (0, 1))))
+    ctx.set_precision(prec, 7)
+    try:
+        _check(ctx, p, tol)
+    finally:
+        ctx.set_precision(lapw1gpu.PREC_FP64)
+
+
+def test_local_orbital_forces_of_many_equivalent_atoms(ctx, many_lo):
+    """Atoms of the first, second and third eight of the type, and one of
+    another type, against the oracle's Hellmann-Feynman sum."""
+    p = many_lo
+    w, _ = FR.eigh(p)
+    nb, _ = FR.gapped_nb(w)
+    atoms = (0, 9, 16, 21)
+    ref = FR.hf_gradient(p, nb, atoms=atoms)
+    occ = torch.ones(nb, dtype=torch.float64, device=torch.device("cuda", ctx.device))
+    ctx.set_precision(lapw1gpu.PREC_FP64)
+    _, eps, X, kp = FO.band_energy(ctx, p, occ)
+    g = FO.gradient(ctx, kp, X, occ, eps).cpu().numpy()
+    kp.free()
+    assert np.abs(g - ref)[list(atoms)].max() <= 1e-8 * np.abs(ref).max()
 
 
 # bands around a tile of 40 (32 at 7 and 8 slices), blocks whose last rows
